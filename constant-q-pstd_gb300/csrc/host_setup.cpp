@@ -12,7 +12,7 @@
 
 #include <initializer_list>
 
-#include "xplans_list.h"
+#include "rt_list.h"
 
 #include <algorithm>
 #include <cmath>
@@ -202,7 +202,7 @@ static void host_fft(std::vector<std::complex<double>>& x, const std::vector<int
         const int nb = n / r;
         for (int j = 0; j < nb; j++) {
             const int k = j % ns;
-            std::complex<double> v[16], o[16];
+            std::complex<double> v[32], o[32];
             for (int q = 0; q < r; q++) {
                 const double ang = sgn * 2.0 * M_PI * (double)(q * k) / (double)(ns * r);
                 v[q] = (*src)[j + q * nb] * std::complex<double>(std::cos(ang), std::sin(ang));
@@ -224,41 +224,39 @@ static void host_fft(std::vector<std::complex<double>>& x, const std::vector<int
     if (src != &x) x = *src;
 }
 
-// Lengths whose x passes are compiled with the plan built in (xplans_list.h):
-// their passes run about a fifth faster than the run-time plan (measured on
-// the z passes), which the planner counts as a lower cost.  Long entries
-// (TX > 0) are the only plans for lines beyond the one-butterfly-per-thread
-// limit.
-struct CompiledPlan {
-    int tx;
-    std::vector<int> rad;
-    int m() const {
-        int v = 1;
-        for (int r : rad) v *= r;
-        return v;
+// Lengths with compiled z passes (ac_kernels.cu, vz_kernels.cu).
+static bool compiled_conv_length(int m) { return m == 200 || m == 660 || m == 1728; }
+
+static RtEntry entry(int id, RtAxis axis, bool quick) {
+    return axis == kRtX ? rt_entry(id, quick) : axis == kRtZ ? rtz_entry(id, quick) : RtEntry{};
+}
+
+int rt_choose(int n, RtAxis axis) {
+    int best = 0;
+    double cost = 1e300;
+    for (int id = 1; id <= std::max(kRtIds, kRtzIds); id++) {
+        const RtEntry e = entry(id, axis, false);
+        if (e.m && (e.pad ? e.m >= 2 * n - 1 : e.m == n) && (double)e.m * e.cost < cost) {
+            cost = (double)e.m * e.cost;
+            best = id;
+        }
     }
-};
-#define QP_XPLAN_ENTRY(TX, ...) CompiledPlan{TX, {__VA_ARGS__}},
-static const std::vector<CompiledPlan>& compiled_plans() {
-    static const std::vector<CompiledPlan> v = {QP_XPLANS_ALL(QP_XPLAN_ENTRY)};
-    return v;
+    return best;
 }
-static const CompiledPlan* compiled_length(int m) {
-    for (const CompiledPlan& c : compiled_plans())
-        if (c.m() == m) return &c;
-    return nullptr;
-}
-static bool compiled_conv_length(int m) {
-    const CompiledPlan* c = compiled_length(m);
-    return c && c->tx == 0;
+
+int rt_lines(int id, RtAxis axis, int quick) { return entry(id, axis, quick != 0).lines; }
+int rt_length(int id, RtAxis axis) { return entry(id, axis, false).m; }
+
+int rt_quick(int id, RtAxis axis, int lines) {
+    const RtEntry w = entry(id, axis, false), q = entry(id, axis, true);
+    return q.m > 0 && (lines + w.lines - 1) / w.lines < 152;
 }
 
 // The smooth lengths m in [2n-1, 2.3n+8] a zero-padded convolution or a
 // Bluestein transform of an n-point line can use, with their radices: the
 // cheapest by pass work (extra_pass: 1 for Bluestein's two transforms per
-// DFT), compiled plans counted at 0.8; with allow_long, a compiled long plan
-// when no length has a one-butterfly-per-thread plan.
-static bool choose_inner_length(int n, bool allow_long, int extra_pass, HostPlan& hp) {
+// DFT), compiled plans counted at 0.8.
+static bool choose_inner_length(int n, int extra_pass, HostPlan& hp) {
     double best = 1e300;
     for (int m = 2 * n - 1; m <= (int)(2.3 * n) + 8; m++) {
         if (!smooth7(m)) continue;
@@ -270,66 +268,50 @@ static bool choose_inner_length(int n, bool allow_long, int extra_pass, HostPlan
             best = cost;
             hp.m = m;
             hp.rad = r;
-            hp.tx = 0;
         }
     }
-    if (best < 1e300 || !allow_long) return best < 1e300;
-    for (int m = 2 * n - 1; m <= (int)(2.3 * n) + 8; m++) {
-        const CompiledPlan* c = compiled_length(m);
-        if (!c || c->tx == 0) continue;
-        hp.m = m;
-        hp.rad = c->rad;
-        hp.tx = c->tx;
-        return true;
-    }
-    return false;
+    return best < 1e300;
 }
 
-int build_plan_host(int n, HostPlan& hp, bool allow_long) {
+static void plan_twiddles(HostPlan& hp) {
+    hp.w.resize(hp.m);
+    for (int k = 0; k < hp.m; k++) {
+        const double a = -2.0 * M_PI * (double)k / (double)hp.m;
+        hp.w[k] = std::complex<double>(std::cos(a), std::sin(a));
+    }
+}
+
+void add_bluestein(HostPlan& hp) {
+    const int n = hp.n, m = hp.m;
+    hp.chirp.resize(n);
+    for (long long k = 0; k < n; k++) {
+        const long long q = (k * k) % (2LL * n);
+        const double a = -M_PI * (double)q / (double)n;
+        hp.chirp[k] = std::complex<double>(std::cos(a), std::sin(a));
+    }
+    std::vector<std::complex<double>> b(m, 0.0);
+    for (int k = 0; k < n; k++) b[k] = std::conj(hp.chirp[k]);
+    for (int k = 1; k < n; k++) b[m - k] = std::conj(hp.chirp[k]);
+    host_fft(b, hp.rad, -1);
+    hp.bhat.resize(m);
+    for (int k = 0; k < m; k++) hp.bhat[k] = b[k] / (double)m;
+}
+
+int build_plan_host(int n, HostPlan& hp) {
+    hp = HostPlan();
     hp.n = n;
-    hp.blue = 0;
-    hp.tx = 0;
     if (n == 1) {
         hp.m = 1;
-        hp.rad.clear();
     } else if (factor_direct(n, hp.rad)) {
         hp.m = n;
     } else {
         // Bluestein: the {2,3,5,7}-smooth inner length in [2n-1, 2.3n] with the
-        // lowest pass work, m * (passes + 1), weighted by radix_weight; for long
-        // lines the compiled long plan the convolution plan of n takes too
+        // lowest pass work, m * (passes + 1), weighted by radix_weight
         hp.blue = 1;
-        if (!choose_inner_length(n, allow_long, 1, hp)) return -1;
-        if (hp.tx > 0) {
-            HostPlan c;
-            if (build_conv_plan_host(n, c, true) || c.tx == 0) return -1;
-            hp.m = c.m;
-            hp.rad = c.rad;
-            hp.tx = c.tx;
-        }
+        if (!choose_inner_length(n, 1, hp)) return -1;
     }
-    const int m = hp.m;
-    hp.w.resize(m);
-    for (int k = 0; k < m; k++) {
-        const double a = -2.0 * M_PI * (double)k / (double)m;
-        hp.w[k] = std::complex<double>(std::cos(a), std::sin(a));
-    }
-    hp.chirp.clear();
-    hp.bhat.clear();
-    if (hp.blue) {
-        hp.chirp.resize(n);
-        for (long long k = 0; k < n; k++) {
-            const long long q = (k * k) % (2LL * n);
-            const double a = -M_PI * (double)q / (double)n;
-            hp.chirp[k] = std::complex<double>(std::cos(a), std::sin(a));
-        }
-        std::vector<std::complex<double>> b(m, 0.0);
-        for (int k = 0; k < n; k++) b[k] = std::conj(hp.chirp[k]);
-        for (int k = 1; k < n; k++) b[m - k] = std::conj(hp.chirp[k]);
-        host_fft(b, hp.rad, -1);
-        hp.bhat.resize(m);
-        for (int k = 0; k < m; k++) hp.bhat[k] = b[k] / (double)m;
-    }
+    plan_twiddles(hp);
+    if (hp.blue) add_bluestein(hp);
     return 0;
 }
 
@@ -338,19 +320,44 @@ int build_plan_host(int n, HostPlan& hp, bool allow_long) {
 // one zero-padded forward and one inverse length-m FFT (every lag i-j in
 // (-n, n) lands on a distinct slot of the length-m wrap), so a window length
 // with a large prime factor costs two smooth FFTs instead of Bluestein's four.
-int build_conv_plan_host(int n, HostPlan& hp, bool allow_long) {
+bool stockham_line(int n) {
+    HostPlan hp;
+    return n == 1 || factor_direct(n, hp.rad) || choose_inner_length(n, 0, hp);
+}
+
+int build_conv_plan_host(int n, HostPlan& hp, RtAxis axis) {
     hp = HostPlan();
     hp.n = n;
-    if (n == 1 || factor_direct(n, hp.rad)) {
-        hp.m = (n == 1) ? 1 : n;
-        if (n == 1) hp.rad.clear();
-    } else if (!choose_inner_length(n, allow_long, 0, hp)) {
+    if ((hp.rt = rt_choose(n, axis)) > 0) {
+        const RtEntry e = entry(hp.rt, axis, false);
+        hp.m = e.m;
+        for (int r : {e.r1, e.r2, e.r3})
+            if (r > 1) hp.rad.push_back(r);
+    } else if (n == 1) {
+        hp.m = 1;
+    } else if (factor_direct(n, hp.rad)) {
+        hp.m = n;
+    } else if (!choose_inner_length(n, 0, hp)) {
         return -1;
     }
-    hp.w.resize(hp.m);
-    for (int k = 0; k < hp.m; k++) {
-        const double a = -2.0 * M_PI * (double)k / (double)hp.m;
-        hp.w[k] = std::complex<double>(std::cos(a), std::sin(a));
+    if (!hp.rt) {
+        plan_twiddles(hp);
+        return 0;
+    }
+    // the tables of the entry's two forms (line_rt.cuh)
+    for (bool quick : {false, true}) {
+        const RtEntry e = entry(hp.rt, axis, quick);
+        if (!e.m) continue;
+        auto put = [&](long long k, int n) {
+            const double a = -2.0 * M_PI * (double)(k % n) / (double)n;
+            hp.w.push_back(std::complex<double>(std::cos(a), std::sin(a)));
+        };
+        for (int r = 0; r < e.r1; r++)
+            for (int j = 0; j < e.m / e.r1; j++) put((long long)r * j, e.m);
+        for (int b = 0; b < e.r2; b++)
+            for (int c = 0; c < e.r3; c++) put((long long)b * c, e.r2 * e.r3);
+        if (hp.w.size() % 2) hp.w.push_back(0.0);  // the kernels copy it in 16-byte pieces
+        if (!quick) hp.wq = (int)hp.w.size();
     }
     return 0;
 }
@@ -397,8 +404,10 @@ int fill_plan_dev(const HostPlan& hp, FFTPlanDev& d) {
         ns *= p.R;
     }
     d.w = d.chirp = d.bhat = nullptr;
-    if (hp.tx > 0) {  // a compiled long plan: TX threads, several butterflies each
-        d.tx = hp.tx;
+    d.rt = hp.rt;
+    d.quick = 0;
+    if (hp.rt) {  // the entry's own thread count
+        d.tx = 32;
         return 0;
     }
     d.tx = std::min(QP_MAXTHREADS, (maxb + 31) / 32 * 32);

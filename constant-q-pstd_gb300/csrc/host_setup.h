@@ -21,16 +21,30 @@ void shift_symbols(int n, double d, int which, std::vector<std::complex<double>>
 
 struct HostPlan {
     int n = 0, m = 0, blue = 0;
-    int tx = 0;  // threads per line of a compiled long plan (0: one butterfly per thread)
+    int rt = 0;  // entry of rt_list.h (0: a Stockham plan of fft_reg.cuh, one butterfly per thread)
+    int wq = 0;  // rt: where the twiddles of the entry's quick form start in w
     std::vector<int> rad;
     std::vector<std::complex<double>> w, chirp, bhat;
 };
-// allow_long: lines that only a compiled long plan (xplans_list.h, group 3)
-// can run may use one; only the x passes have those kernels.
-int build_plan_host(int n, HostPlan& hp, bool allow_long = false);
+// Exact DFT plan of a Stockham pass: n itself when it factors into radices <= 16,
+// else Bluestein on a smooth m >= 2n-1.
+int build_plan_host(int n, HostPlan& hp);
 // Length-m FFT plan for separable operators applied as zero-padded circular
-// convolutions (m = n when n factors into radices <= 16, else smooth m >= 2n-1).
-int build_conv_plan_host(int n, HostPlan& hp, bool allow_long = false);
+// convolutions.  On an entry of rt_list.h's x or z passes (axis), where one is long
+// enough; else (or for kStockham) a Stockham plan, m = n when n factors into radices
+// <= 16, else a smooth m >= 2n-1.
+enum RtAxis { kStockham, kRtX, kRtZ };
+int build_conv_plan_host(int n, HostPlan& hp, RtAxis axis = kStockham);
+// Is there a Stockham plan for an n-point line?
+bool stockham_line(int n);
+// Adds the tables of the exact length-n DFT by Bluestein's identity on hp.m.
+void add_bluestein(HostPlan& hp);
+// The entry of rt_list.h an n-point line runs on (0: none is long enough), whether
+// it runs the entry's quick form for this number of lines, and its lines per CTA.
+int rt_choose(int n, RtAxis axis);
+int rt_quick(int id, RtAxis axis, int lines);
+int rt_lines(int id, RtAxis axis, int quick);
+int rt_length(int id, RtAxis axis);
 // Length-m multiplier of the convolution form of the symbol Hn (1/n folded in).
 void conv_table(const HostPlan& hp, const std::vector<std::complex<double>>& Hn,
                 std::vector<std::complex<double>>& out);

@@ -104,7 +104,7 @@ const float* put_real(TableImage& im, const std::vector<double>& v) {
 // not fit the static array.
 int put_plan(TableImage& im, const HostPlan& hp, FFTPlanDev& pd) {
     int maxb = 1;
-    for (int r : hp.rad) maxb = std::max(maxb, hp.m / r);
+    if (!hp.rt) for (int r : hp.rad) maxb = std::max(maxb, hp.m / r);
     if (maxb > QP_MAXTHREADS)
         return fail(QPSTD_ENOTSUP, "transform needs more threads per line than a CTA holds");
     const float2* tw = put_complex(im, hp.w);
@@ -124,7 +124,10 @@ int put_plan(TableImage& im, const HostPlan& hp, FFTPlanDev& pd) {
         ns *= q.R;
     }
     pd.tx = (maxb + 31) / 32 * 32;
+    pd.rt = hp.rt;
+    pd.quick = 0;
     pd.w = tw;
+    pd.wq = tw + hp.wq;
     pd.chirp = pd.bhat = nullptr;
     return QPSTD_OK;
 }
@@ -190,10 +193,18 @@ extern "C" int qpstd_ac_advance_noalloc(const qpstd_shot_desc* d, const float* v
     HostPlan cx, cz;
     if (build_conv_plan_host(nxx, cx) || build_conv_plan_host(nzz, cz))
         return fail(QPSTD_ENOTSUP, "no convolution plan for this length");
+    if (rt_choose(nxx, kRtX) && rt_choose(nzz, kRtZ)) {  // on the register-to-register passes
+        build_conv_plan_host(nxx, cx, kRtX);
+        build_conv_plan_host(nzz, cz, kRtZ);
+    }
     FFTPlanDev px{}, pz{};
     int prc = put_plan(im, cx, px);
     if (prc == QPSTD_OK) prc = put_plan(im, cz, pz);
     if (prc != QPSTD_OK) return prc;
+    if (px.rt) {
+        set_quick(px, rt_quick(px.rt, kRtX, (nzz + 1) / 2));
+        set_quick(pz, rt_quick(pz.rt, kRtZ, (nxx + 1) / 2));
+    }
     std::vector<std::complex<double>> H, T;
     const float2* tab[6];  // x velocity, x pressure, z velocity, z pressure derivatives; kx^2; kz^2
     for (int w = 0; w < 4; w++) {
@@ -223,11 +234,11 @@ extern "C" int qpstd_ac_advance_noalloc(const qpstd_shot_desc* d, const float* v
 
     // tile shapes and staging as qpstd_shot_create chooses them
     const size_t stz = (size_t)40 * nzz, stx = (size_t)72 * nxx;
-    const bool stage_z = ((size_t)8 * pz.m + stz) <= (size_t)QP_SMEM_DYN_MAX;
-    const bool stage_x = ((size_t)8 * px.m + stx) <= (size_t)QP_SMEM_DYN_MAX;
-    const int Lx = lines_per_cta((nzz + 1) / 2, px, stage_x ? stx : 0,
+    const bool stage_z = !pz.rt && ((size_t)8 * pz.m + stz) <= (size_t)QP_SMEM_DYN_MAX;
+    const bool stage_x = !px.rt && ((size_t)8 * px.m + stx) <= (size_t)QP_SMEM_DYN_MAX;
+    const int Lx = px.rt ? rt_lines(px.rt, kRtX, px.quick) : lines_per_cta((nzz + 1) / 2, px, stage_x ? stx : 0,
                                  stage_x ? (size_t)QP_SMEM_DYN_MAX : 160 * 1024, true);
-    int Lzp = lines_per_cta((nxx + 1) / 2, pz, stage_z ? stz : 0, 110 * 1024, false);
+    int Lzp = pz.rt ? 1 : lines_per_cta((nxx + 1) / 2, pz, stage_z ? stz : 0, 110 * 1024, false);
     if (stage_z && (size_t)8 * pz.m + stz > 110 * 1024) Lzp = 1;
 
     // receivers grouped by x-pass tile; per cell the highest index injects
@@ -270,6 +281,7 @@ extern "C" int qpstd_ac_advance_noalloc(const qpstd_shot_desc* d, const float* v
         a.i_az = pm[2]; a.i_bz = pm[3]; a.h_az = pm[6]; a.h_bz = pm[7];
         a.bbz = bbz; a.p = p; a.vz = vz; a.psi_pz = fipz; a.psi_vz = fivzz; a.Dx = Dx;
         a.div = div; a.Lz = Lzf; a.dt = d->dt; a.do_v = do_v; a.do_div = do_div; a.stage = stage_z;
+        a.rs = a.rz = nzz; a.sb = 4;
         return a;
     };
     auto xargs = [&](int do_p, int do_v, int do_dx) {
@@ -280,6 +292,7 @@ extern "C" int qpstd_ac_advance_noalloc(const qpstd_shot_desc* d, const float* v
         a.bbx = bbx; a.c1 = c1; a.c2 = c2; a.p = p; a.vx = vx; a.psi_px = fipx; a.psi_vx = fivxx; a.Dx = Dx;
         a.div = div; a.Lz = Lzf; a.dt = d->dt; a.do_p = do_p; a.do_v = do_v; a.do_dx = do_dx;
         a.xs = -1; a.zs = -1; a.stage = stage_x;
+        a.rs = nzz; a.sb = 4;
         return a;
     };
     launch_ac_xpass(xargs(0, 0, 1), st);

@@ -159,4 +159,30 @@ __device__ __forceinline__ void xfill(float* sf, const XTile& T, int ld, Get&& g
         });
 }
 
+// The isotropic symbols of the x-spectral passes at squared wavenumber k2: output j of
+// mode 0, the one of mode 1, the stabilised Q-RTM filter of mode 2.
+__device__ __forceinline__ float spec_symbol(const VxsArgs& a, int j, float k2) {
+    if (a.mode == 0) {
+        if (j == 1) return k2;
+        const float k32 = exp2f(log2f(k2) * (1.f / 32.f));
+        return (j == 0) ? k32 : k2 * k32;
+    }
+    const float ka = exp2f(0.505f * log2f(k2));
+    if (a.mode == 1) return ka;
+    const float num = 2.f * a.eta6 * ka * (1.f + a.tao * a.dt * ka);
+    const float den = expf(-a.tao * a.tt * ka) + a.eta6 * expf(a.tao * a.dt * ka);
+    return ka - num / den;
+}
+// The stationary symbols of the convolution tables in double (see VtabArgs).
+__device__ __forceinline__ double tab_symbol(const VtabArgs& a, int kx, int kz, double k2) {
+    if (a.sym == 4) {
+        const int hx = (kx < a.nxh) ? kx : a.nxx - kx, hz = min(kz, a.nzz - kz);
+        return a.V[(size_t)hx * (a.nzz / 2 + 1) + hz];
+    }
+    if (a.sym == 1) return k2;
+    if (a.sym == 0) return pow(k2, 1.0 / 32.0);
+    if (a.sym == 2) return pow(k2, 33.0 / 32.0);
+    return pow(k2, 0.505);
+}
+
 }  // namespace qp

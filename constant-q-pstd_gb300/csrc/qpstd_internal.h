@@ -43,11 +43,20 @@ struct FFTPlanDev {
     int blue;              // 1 if Bluestein is used
     int nst;               // number of passes of the length-m transform
     int tx;                // threads per line (>= max B, multiple of 32)
+    int rt;                // entry of rt_list.h whose register-to-register passes run this plan (0: none)
+    int quick;             // 1: the entry's one-line-per-CTA form
     FFTPass pass[QP_MAXST];
-    const float2* w;       // m twiddles e^{-2 pi i k/m}
+    const float2* w;       // m twiddles e^{-2 pi i k/m}; rt: the tables of line_rt.cuh
+    const float2* wq;      // rt: the same of the quick form
     const float2* chirp;   // n chirp values e^{-i pi k^2/n} (Bluestein)
     const float2* bhat;    // m values: DFT_m of the wrapped conj chirp, divided by m (Bluestein)
 };
+
+// Runs the quick (1) or the wide (0) form of an rt plan.
+inline void set_quick(FFTPlanDev& p, int quick) {
+    p.quick = quick;
+    if (quick) p.w = p.wq;
+}
 
 // Largest radix of a plan (host or device): kernels with plans up to radix 12
 // can run the 12-entry register array.
@@ -84,6 +93,7 @@ struct AcZArgs {
     float dt;
     int do_v, do_div;
     int stage;                    // stage epilogue inputs in shared memory (cp.async)
+    unsigned rs, sb, rz;          // rt: strides of the fields (rt_z.cuh)
 };
 
 // ---------------------------------------------------------------------------
@@ -130,6 +140,8 @@ struct AcXArgs {
     float *ssg, *ssg_c;           // illumination accumulation, Kahan pair (NULL: off)
     float *img, *img_c;           // image accumulation, Kahan pair (NULL: off)
     const float* ps;              // source wavefield p for imaging
+    int vec;                      // rt: rows of a tile are aligned for one vector access
+    unsigned rs, sb;              // rt: strides of the fields (rt_z.cuh); ssg and img have them too
     int stage;                    // stage epilogue inputs in shared memory (cp.async)
 };
 
@@ -156,6 +168,7 @@ struct VzArgsA {
     const float* Dx;
     float* div;
     float2* G;
+    unsigned rs, sb, rz, srs, ssb;  // rt: strides of the fields and the half spectra (rt_z.cuh)
 };
 
 // x pass over half spectra: out_j = F_x^-1[ sym_j(kx,kz) F_x in ] / (nxx nzz).
@@ -173,6 +186,7 @@ struct VxsArgs {
     float norm;               // 1/(nxx*nzz)
     float eta6;               // eta * 1e-6 (mode 2)
     float tao, dt, tt;        // filter tau, dt, nt*dt (mode 2)
+    unsigned srs, ssb;        // rt: strides of the half spectra
 };
 
 // Builds the per-kz convolution multipliers of a stationary 2-D symbol:
@@ -184,7 +198,7 @@ struct VtabArgs {
                                 //      4 the low-rank factor V (half grid, mirrored in kx)
     FFTPlanDev pl, plc;
     const float *kx2, *kz2;
-    const float* V;             // sym 4: nxh x nzh values of one factor
+    const float* V;             // sym 4: nxh x (nzz/2+1) values of one factor
     int nxh;
     float norm;
     float* out;
@@ -201,13 +215,26 @@ struct LrxArgs {
     float2* out;                // row half spectra, factor-major (b * nxx * nzh)
     const float* tab;           // row x nzh x (plc.m/2+1)
 };
+// rt: out_b = F_x^-1[tab_b F_x in] for nout tables tab + b tab_step and outputs
+// out + b out_step (modes 0 and 1 of VxsArgs, and LrxArgs).
+struct XconvArgs {
+    int nxx, nzh, nout;
+    FFTPlanDev pl;
+    const float2* in;
+    const float* tab;
+    float2* out;
+    size_t tab_step, out_step;
+    unsigned srs, ssb;          // strides of the half spectra
+};
 // z pass: psc(x) = sum_b c_b(x) Re F_z^-1[Q_b](x), c_b(x) = sum_a U[x][a] A[a][b].
 struct LrsArgs {
     int nxx, nzz, nzh, L, row;
     FFTPlanDev pl;              // exact length-nzz plan
     const float2* Q;
-    const float* c;             // row x nxx*nzz
+    const float* c;             // row x npts (rt: null for the field of one spectrum itself)
     float* psc;
+    size_t npts;                // points of a field (rt: with its padding)
+    unsigned rs, sb, rz, srs, ssb;  // rt: strides of the fields and the half spectra
 };
 
 // z pass B: Y2, Y3, Y4 from their spectra; total; total -> half spectrum T.
@@ -219,6 +246,7 @@ struct VzArgsB {
     const float *y1, *y2, *y3c, *y4c;
     float* total;
     float2* T;
+    unsigned rs, sb, rz, srs, ssb;  // rt: strides of the fields and the half spectra
 };
 
 // z pass C: D from its spectrum; pressure update (+ source, receivers,
@@ -245,6 +273,7 @@ struct VzArgsC {
     const float *h_az, *h_bz, *bbz;
     float *vz, *psi_pz;
     float dt;
+    unsigned rs, sb, rz, srs, ssb;  // rt: strides (ssg, img too)
 };
 
 // z pass that only turns a half spectrum back into a real field.

@@ -1,0 +1,94 @@
+// rt_list.h -- the line lengths compiled into the register-to-register passes
+// (line_rt.cuh), host and device view.
+//
+// x entries are X(ID, W, G, MB, R1, R2, R3, COST): W complex lines per thread, G groups of W
+// lines per CTA, MB CTAs per SM the kernels are compiled for, the radices, and the measured
+// clocks x 1000 per point and roundtrip of one SM (a batch of full SMs).  All of them serve
+// zero-padded lines: an n-point line runs on the entry of length M >= 2n - 1 with the least
+// M x COST.  Radices of powers of two cost least, so the ladder is dense around them: lengths
+// between two entries would cost as much as the next one (900 = 30 x 30: 0.93, 1024 = 32 x 32:
+// 0.73 clocks; 3840: 0.99, 4096: 0.93).  Up to 1024 two passes of radices up to 32 with one
+// line per thread beat three (900: 0.93 against 1.05); above, three passes with two packed
+// lines beat one line (3360: 1.07 against 1.22); beyond 4608 two lines leave no registers
+// for a second CTA (5120: 1.19 against 1.14).
+//
+// z entries are X(ID, W, PAD, GF, G, MB, R1, R2, R3, COST): PAD 0 transforms lines of exactly
+// M points, PAD 1 serves n <= (M + 1) / 2 (operators as padded convolutions, exact DFTs by
+// Bluestein's identity).  GF 1: a warp's threads are neighbouring rows, whose points are
+// neighbours in the blocked fields.
+//
+// The wide forms fill the chip with many lines; the quick forms have the same lengths with
+// fewer lines per CTA on more threads, for grids whose wide form has fewer CTAs than the
+// chip has SMs (there the latency of one line counts).
+#pragma once
+
+// Each group is compiled by itself (rt_group.cu), to keep the build parallel.
+#define QP_RT_G0(X) X(1, 2, 8, 4, 10, 1, 16, 650) X(2, 2, 8, 3, 16, 1, 16, 500) X(3, 2, 2, 5, 8, 6, 8, 800)
+#define QP_RT_G1(X) X(4, 2, 2, 4, 8, 8, 8, 760) X(5, 2, 1, 5, 8, 12, 8, 850)
+#define QP_RT_G2(X) X(6, 2, 1, 4, 8, 16, 8, 820) X(7, 2, 1, 4, 16, 8, 10, 980)
+#define QP_RT_G3(X) X(8, 2, 1, 3, 16, 8, 12, 1000) X(9, 2, 1, 4, 16, 8, 16, 950)
+#define QP_RT_G4(X) X(10, 2, 1, 2, 16, 12, 12, 1060) X(11, 2, 1, 3, 16, 10, 16, 1080)
+#define QP_RT_G5(X) X(12, 2, 1, 2, 16, 12, 16, 1050) X(13, 2, 1, 2, 16, 14, 15, 1070)
+#define QP_RT_G6(X) X(14, 2, 1, 2, 16, 16, 16, 930) X(15, 1, 1, 2, 16, 20, 16, 1140)
+#define QP_RT_G7(X) X(16, 1, 1, 1, 24, 16, 16, 1400) X(17, 1, 1, 1, 20, 18, 20, 1470)
+#define QP_RT_G8(X) X(18, 1, 1, 1, 24, 18, 20, 1460) X(19, 1, 1, 1, 24, 16, 24, 1460)
+#define QP_RT_G9(X) X(1, 1, 1, 8, 10, 1, 16, 0) X(2, 1, 1, 8, 16, 1, 16, 0) X(3, 1, 1, 8, 8, 6, 8, 0) X(4, 1, 1, 8, 8, 8, 8, 0) X(5, 1, 1, 6, 8, 12, 8, 0)
+#define QP_RT_G10(X) X(6, 1, 1, 5, 8, 16, 8, 0) X(7, 1, 1, 4, 8, 16, 10, 0) X(8, 1, 1, 4, 8, 16, 12, 0)
+#define QP_RT_G11(X) X(9, 1, 1, 4, 8, 16, 16, 0) X(10, 1, 1, 3, 12, 12, 16, 0) X(11, 1, 1, 3, 16, 10, 16, 0)
+#define QP_RT_G12(X) X(12, 1, 1, 3, 16, 12, 16, 0) X(13, 1, 1, 3, 16, 14, 15, 0) X(14, 1, 1, 3, 16, 16, 16, 0)
+#define QP_RTZ_G0(X) X(1, 1, 0, 1, 8, 4, 15, 1, 12, 1000) X(2, 1, 0, 1, 8, 3, 10, 1, 20, 1110) X(3, 1, 0, 1, 8, 4, 16, 1, 16, 700)
+#define QP_RTZ_G1(X) X(4, 1, 0, 1, 4, 4, 8, 5, 8, 1100) X(5, 1, 0, 1, 4, 3, 10, 5, 8, 1200) X(6, 1, 0, 1, 2, 5, 8, 8, 8, 1050)
+#define QP_RTZ_G2(X) X(7, 1, 0, 1, 2, 4, 8, 8, 10, 1150) X(8, 1, 0, 1, 2, 4, 11, 6, 10, 1600)
+#define QP_RTZ_G3(X) X(9, 1, 0, 1, 2, 4, 10, 8, 10, 1250) X(15, 1, 1, 1, 2, 2, 8, 16, 8, 1000)
+#define QP_RTZ_G4(X) X(10, 1, 1, 1, 8, 4, 10, 1, 16, 800) X(11, 1, 1, 1, 8, 4, 16, 1, 16, 600) X(12, 1, 1, 1, 4, 3, 8, 6, 8, 1000)
+#define QP_RTZ_G5(X) X(13, 1, 1, 1, 2, 5, 8, 8, 8, 950) X(14, 1, 1, 1, 2, 3, 8, 12, 8, 1050)
+#define QP_RTZ_G6(X) X(16, 1, 1, 1, 2, 2, 16, 8, 10, 1200) X(17, 1, 1, 1, 2, 2, 16, 8, 12, 1200)
+#define QP_RTZ_G7(X) X(18, 1, 1, 1, 2, 2, 16, 8, 16, 1150) X(19, 1, 1, 0, 1, 3, 16, 12, 12, 1250)
+#define QP_RTZ_G8(X) X(20, 1, 1, 0, 1, 4, 16, 10, 16, 1250) X(21, 1, 1, 0, 1, 3, 16, 12, 16, 1250)
+#define QP_RTZ_G9(X) X(22, 1, 1, 0, 1, 2, 16, 16, 16, 1150) X(23, 1, 1, 0, 1, 2, 16, 20, 16, 1140)
+#define QP_RTZ_G10(X) X(24, 1, 1, 0, 1, 1, 24, 16, 16, 1400)
+#define QP_RTZ_G11(X) X(1, 1, 0, 0, 1, 4, 15, 1, 12, 0) X(2, 1, 0, 0, 1, 4, 10, 1, 20, 0) X(3, 1, 0, 0, 1, 4, 16, 1, 16, 0) X(4, 1, 0, 0, 1, 4, 8, 5, 8, 0) X(5, 1, 0, 0, 1, 4, 10, 5, 8, 0)
+#define QP_RTZ_G12(X) X(6, 1, 0, 0, 1, 4, 8, 8, 8, 0) X(7, 1, 0, 0, 1, 4, 8, 8, 10, 0) X(8, 1, 0, 0, 1, 4, 11, 6, 10, 0) X(9, 1, 0, 0, 1, 4, 10, 8, 10, 0)
+#define QP_RTZ_G13(X) X(10, 1, 1, 0, 1, 4, 10, 1, 16, 0) X(11, 1, 1, 0, 1, 4, 16, 1, 16, 0) X(12, 1, 1, 0, 1, 4, 8, 6, 8, 0) X(13, 1, 1, 0, 1, 4, 8, 8, 8, 0)
+#define QP_RTZ_G14(X) X(14, 1, 1, 0, 1, 4, 8, 12, 8, 0) X(15, 1, 1, 0, 1, 4, 8, 16, 8, 0)
+#define QP_RT_WIDE_ALL(X) \
+    QP_RT_G0(X) QP_RT_G1(X) QP_RT_G2(X) QP_RT_G3(X) QP_RT_G4(X) QP_RT_G5(X) QP_RT_G6(X) QP_RT_G7(X) QP_RT_G8(X)
+#define QP_RT_QUICK_ALL(X) \
+    QP_RT_G9(X) QP_RT_G10(X) QP_RT_G11(X) QP_RT_G12(X)
+#define QP_RTZ_WIDE_ALL(X) \
+    QP_RTZ_G0(X) QP_RTZ_G1(X) QP_RTZ_G2(X) QP_RTZ_G3(X) QP_RTZ_G4(X) QP_RTZ_G5(X) QP_RTZ_G6(X) QP_RTZ_G7(X) QP_RTZ_G8(X) QP_RTZ_G9(X) QP_RTZ_G10(X)
+#define QP_RTZ_QUICK_ALL(X) \
+    QP_RTZ_G11(X) QP_RTZ_G12(X) QP_RTZ_G13(X) QP_RTZ_G14(X)
+// groups of the wide forms come first
+#define QP_RT_NWIDE 9
+#define QP_RT_NGROUPS 13
+#define QP_RTZ_NWIDE 11
+#define QP_RTZ_NGROUPS 15
+
+// An entry's complex lines per CTA, length and radices (m = 0: no such entry).
+struct RtEntry {
+    int lines, m, pad, cost, r1, r2, r3;
+};
+inline RtEntry rt_entry(int id, bool quick) {
+#define QP_RT_CASE(ID, W, G, MB, R1, R2, R3, COST) \
+    if (id == ID) return {W * G, R1 * R2 * R3, 1, COST, R1, R2, R3};
+    if (quick) {
+        QP_RT_QUICK_ALL(QP_RT_CASE)
+    } else {
+        QP_RT_WIDE_ALL(QP_RT_CASE)
+    }
+#undef QP_RT_CASE
+    return {0, 0, 0, 0, 0, 0, 0};
+}
+inline RtEntry rtz_entry(int id, bool quick) {
+#define QP_RT_CASE(ID, W, PAD, GF, G, MB, R1, R2, R3, COST) \
+    if (id == ID) return {W * G, R1 * R2 * R3, PAD, COST, R1, R2, R3};
+    if (quick) {
+        QP_RTZ_QUICK_ALL(QP_RT_CASE)
+    } else {
+        QP_RTZ_WIDE_ALL(QP_RT_CASE)
+    }
+#undef QP_RT_CASE
+    return {0, 0, 0, 0, 0, 0, 0};
+}
+constexpr int kRtIds = 19, kRtzIds = 24;

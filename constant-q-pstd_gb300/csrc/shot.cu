@@ -36,6 +36,7 @@ void launch_vz_xspec_conv(const VxsArgs& a, cudaStream_t s);
 void launch_vz_convtab(const VtabArgs& a, cudaStream_t s);
 void launch_lr_xconv(const LrxArgs& a, cudaStream_t s);
 void launch_lr_zsum(const LrsArgs& a, cudaStream_t s);
+void launch_rt_xconv(const XconvArgs& a, cudaStream_t s);
 int vz_set_smem_limits();
 }  // namespace qp
 
@@ -89,6 +90,58 @@ cudaError_t shot_malloc(qpstd_shot* s, void** p, size_t bytes) {
     return cudaSuccess;
 }
 
+// Host memory to the device on the shot's stream (h may be reused on return: the
+// runtime stages pageable memory).
+static cudaError_t upload(qpstd_shot* s, void* dst, const void* h, size_t bytes) {
+    return cudaMemcpyAsync(dst, h, bytes, cudaMemcpyHostToDevice, s->stream);
+}
+
+// ---- the shot's field layout ---------------------------------------------------------
+// When both directions run the register-to-register passes (s->blk), the fields that the x
+// passes touch are blocked: point (ix, iz) at ix rs + (iz / 4) sb + iz % 4, rs = 4, sb = 4 nxx
+// (rt_z.cuh).  The z passes' own fields, and every field of other shots, lie row by row like
+// the caller's arrays.  The conversions copy a window of nx x nz points at (x0, z0).
+__global__ void field_in_kernel(int nx, int nz, unsigned rs, unsigned sb, const float* __restrict__ in, float* __restrict__ f) {
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (unsigned)nx * nz) return;
+    const unsigned ix = i / nz, iz = i - ix * nz;
+    f[ix * rs + (iz >> 2) * sb + (iz & 3)] = in[i];
+}
+__global__ void field_out_kernel(int nx, int nz, int x0, int z0, unsigned rs, unsigned sb, const float* __restrict__ f,
+                                 float* __restrict__ out) {
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (unsigned)nx * nz) return;
+    const unsigned ix = i / nz, iz = i - ix * nz + z0;
+    out[i] = f[(ix + x0) * rs + (iz >> 2) * sb + (iz & 3)];
+}
+// address of point (ix, iz) of a field the x passes touch
+static size_t field_at(const qpstd_shot* s, int ix, int iz) { return (size_t)ix * s->rs + (size_t)(iz >> 2) * s->sb + (iz & 3); }
+// state fields (p, vx, vz, fipx, fipz, fivxx, fivzz, aux) the x passes touch
+static bool state_blocked(const qpstd_shot* s, int k) { return s->blk && (k == 0 || k == 1 || k == 3 || k == 5); }
+
+// One field of the caller's (nxx * nzz floats) to the device field f, and the window of nx x nz
+// points at (x0, z0) of f back; blocked: f lies blocked.
+static int put_field(qpstd_shot* s, const float* h, float* f, bool blocked) {
+    const size_t n = (size_t)s->d.nxx * s->d.nzz;
+    CK(upload(s, blocked ? s->io : f, h, sizeof(float) * n));
+    if (blocked) {
+        field_in_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(s->d.nxx, s->d.nzz, s->rs, s->sb, s->io, f);
+        CK(cudaGetLastError());
+    }
+    return QPSTD_OK;
+}
+static int get_window(qpstd_shot* s, const float* f, bool blocked, int nx, int nz, int x0, int z0, float* h) {
+    const size_t n = (size_t)nx * nz;
+    if (blocked || nx != s->d.nxx || nz != s->d.nzz) {
+        field_out_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(nx, nz, x0, z0, blocked ? s->rs : s->d.nzz,
+                                                                              blocked ? s->sb : 4, f, s->io);
+        CK(cudaGetLastError());
+        f = s->io;
+    }
+    CK(cudaMemcpyAsync(h, f, sizeof(float) * n, cudaMemcpyDeviceToHost, s->stream));
+    return QPSTD_OK;
+}
+
 static int upload_plan(qpstd_shot* s, const HostPlan& hp, FFTPlanDev& d) {
     if (fill_plan_dev(hp, d)) return fail(QPSTD_ENOTSUP, "transform needs more threads per line than a CTA holds");
     std::vector<float2> h;
@@ -96,10 +149,11 @@ static int upload_plan(qpstd_shot* s, const HostPlan& hp, FFTPlanDev& d) {
     const size_t cnt = h.size();
     float2* dptr = nullptr;
     CK(shot_malloc(s, (void**)&dptr, sizeof(float2) * cnt));
-    CK(cudaMemcpy(dptr, h.data(), sizeof(float2) * cnt, cudaMemcpyHostToDevice));
+    CK(upload(s, dptr, h.data(), sizeof(float2) * cnt));
     d.w = dptr;
-    d.chirp = hp.blue ? dptr + hp.w.size() : nullptr;
-    d.bhat = hp.blue ? dptr + hp.w.size() + hp.chirp.size() : nullptr;
+    d.wq = dptr + hp.wq;
+    d.chirp = hp.chirp.empty() ? nullptr : dptr + hp.w.size();
+    d.bhat = hp.bhat.empty() ? nullptr : dptr + hp.w.size() + hp.chirp.size();
     return QPSTD_OK;
 }
 
@@ -166,11 +220,11 @@ static int build_rec_list(qpstd_shot* s, const qpstd_shot_desc* d, int width, bo
     off[ntile] = (int)flat.size();
     int* doff = nullptr;
     CK(shot_malloc(s, (void**)&doff, sizeof(int) * off.size()));
-    CK(cudaMemcpy(doff, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice));
+    CK(upload(s, doff, off.data(), sizeof(int) * off.size()));
     RecEntry* drec = nullptr;
     const size_t nrec = std::max<size_t>(flat.size(), 1);
     CK(shot_malloc(s, (void**)&drec, sizeof(RecEntry) * nrec));
-    if (!flat.empty()) CK(cudaMemcpy(drec, flat.data(), sizeof(RecEntry) * flat.size(), cudaMemcpyHostToDevice));
+    if (!flat.empty()) CK(upload(s, drec, flat.data(), sizeof(RecEntry) * flat.size()));
     *off_out = doff;
     *rec_out = drec;
     return QPSTD_OK;
@@ -184,32 +238,35 @@ static int build_receivers(qpstd_shot* s, const qpstd_shot_desc* d) {
 
 // Per-point constant-Q coefficients and the spectra scratch (double -> float once).
 static int setup_visco(qpstd_shot* s, const qpstd_shot_desc* d) {
-    const size_t N = s->N;
+    const size_t N = s->N, Nu = (size_t)d->nxx * d->nzz;
     int rc = QPSTD_OK;
     const size_t NS = (size_t)d->nxx * s->nzh;  // half-spectrum length (complex)
     float* f = dalloc(s, 8 * N, &rc);
     if (!f) return rc;
+    CK(cudaMemsetAsync(f, 0, sizeof(float) * 8 * N, s->stream));
     s->y1 = f; s->y2 = f + N; s->y3c = f + 2 * N; s->y4c = f + 3 * N;
     s->e1 = f + 4 * N; s->e2 = f + 5 * N; s->e3 = f + 6 * N; s->total = f + 7 * N;
     float* sp = dalloc(s, 2 * NS * (s->rtm ? 6 : 5), &rc);
     if (!sp) return rc;
+    CK(cudaMemsetAsync(sp, 0, sizeof(float) * 2 * NS * (s->rtm ? 6 : 5), s->stream));
     for (int k = 0; k < 4; k++) s->spec[k] = reinterpret_cast<float2*>(sp) + k * NS;
     s->src.aux_spec = reinterpret_cast<float2*>(sp) + 4 * NS;
     if (s->rtm) s->rcv.aux_spec = reinterpret_cast<float2*>(sp) + 5 * NS;
-    std::vector<float> h(7 * N);
+    std::vector<float> h(7 * Nu);
     const double dt = d->dt;
-    for (size_t i = 0; i < N; i++) {
+    for (size_t i = 0; i < Nu; i++) {
         const double g = d->gam[i], w = d->vwd[i], vp = d->vp[i], lam = d->lam[i], tao = d->tao[i];
         const double cc = dt * dt * vp * vp * lam / 12.0;  // sum_total, acsglw.cu:1213-1245
         h[i] = (float)(1.0 - 32.0 * g);
-        h[N + i] = (float)(32.0 * g * w);
-        h[2 * N + i] = (float)((1.0 - 64.0 * g) * cc);
-        h[3 * N + i] = (float)(64.0 * g * w * cc);
-        h[4 * N + i] = (float)((double)d->rho[i] * vp * vp * dt * lam);  // addsa_kernel, acsglw.cu:1527
-        h[5 * N + i] = (float)(0.5 * dt * tao);
-        h[6 * N + i] = (float)(dt * tao);
+        h[Nu + i] = (float)(32.0 * g * w);
+        h[2 * Nu + i] = (float)((1.0 - 64.0 * g) * cc);
+        h[3 * Nu + i] = (float)(64.0 * g * w * cc);
+        h[4 * Nu + i] = (float)((double)d->rho[i] * vp * vp * dt * lam);  // addsa_kernel, acsglw.cu:1527
+        h[5 * Nu + i] = (float)(0.5 * dt * tao);
+        h[6 * Nu + i] = (float)(dt * tao);
     }
-    CK(cudaMemcpy(f, h.data(), sizeof(float) * 7 * N, cudaMemcpyHostToDevice));
+    for (int k = 0; k < 7; k++)
+        if ((rc = put_field(s, h.data() + (size_t)k * Nu, f + (size_t)k * N, false))) return rc;
     return QPSTD_OK;
 }
 
@@ -227,19 +284,20 @@ static int setup_ksq(qpstd_shot* s, const qpstd_shot_desc* d) {
     }
     float* kk = dalloc(s, k2.size(), &rc);
     if (!kk) return rc;
-    CK(cudaMemcpy(kk, k2.data(), sizeof(float) * k2.size(), cudaMemcpyHostToDevice));
+    CK(upload(s, kk, k2.data(), sizeof(float) * k2.size()));
     s->kxsq = kk;
     s->kzsq = kk + d->nxx;
     return QPSTD_OK;
 }
 
-// Convolution tables of the stationary constant-Q symbols.  When nxx is not a
-// smooth length the exact x transforms of the x-spectral passes go through
-// Bluestein (two FFTs each); a symbol that does not change in time is instead
-// applied per kz column as a circular convolution along x on the smooth
-// convolution length (one FFT per output after a shared forward FFT).
+// Convolution tables of the stationary constant-Q symbols: a symbol that does
+// not change in time is applied per kz column as a circular convolution along x
+// on the convolution length (one FFT per output after a shared forward FFT),
+// which the register-to-register passes run for every width they plan; Stockham
+// plans do so when nxx is not a smooth length, where the exact transforms would
+// go through Bluestein (two FFTs each).
 static int setup_xtabs(qpstd_shot* s, const qpstd_shot_desc* d) {
-    if (!s->px.blue) return QPSTD_OK;
+    if (!s->px.blue && !s->pxc.rt) return QPSTD_OK;
     int rc = QPSTD_OK;
     const int mc = s->pxc.m, nzh = s->nzh, mh = mc / 2 + 1;  // rows keep the even half
     float* t = dalloc(s, (size_t)4 * nzh * mh, &rc);
@@ -248,7 +306,7 @@ static int setup_xtabs(qpstd_shot* s, const qpstd_shot_desc* d) {
     a.nxx = d->nxx; a.nzz = d->nzz; a.nzh = nzh;
     a.pl = s->px; a.plc = s->pxc; a.kx2 = s->kxsq; a.kz2 = s->kzsq;
     a.norm = (float)(1.0 / ((double)d->nxx * d->nzz));
-    a.L = choose_L(nzh, std::max(s->px.m, mc), std::max(s->px.tx, s->pxc.tx), 1, false);
+    if (!s->pxc.rt) a.L = choose_L(nzh, std::max(s->px.m, mc), std::max(s->px.tx, s->pxc.tx), 1, false);
     for (int k = 0; k < 4; k++) {
         a.sym = k;
         a.out = t + (size_t)k * nzh * mh;
@@ -259,6 +317,7 @@ static int setup_xtabs(qpstd_shot* s, const qpstd_shot_desc* d) {
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "convolution tables");
     s->xconv = true;
+    if (s->pxc.rt) return QPSTD_OK;
     s->Lxs_exact = s->Lxs;
     s->Lxs = choose_L(nzh, mc, s->pxc.tx, 1, true);
     s->Lxs3 = choose_L(nzh, mc, s->pxc.tx, 2, true);
@@ -283,7 +342,7 @@ static int setup_plain(qpstd_shot* s, const qpstd_shot_desc* d) {
         *dst[w] = cbase + q;
         for (auto& c : H) hc[q++] = make_float2((float)c.real(), (float)c.imag());
     }
-    CK(cudaMemcpy(cbase, hc.data(), sizeof(float2) * nc, cudaMemcpyHostToDevice));
+    CK(upload(s, cbase, hc.data(), sizeof(float2) * nc));
     return QPSTD_OK;
 }
 
@@ -291,8 +350,11 @@ static int setup_plain(qpstd_shot* s, const qpstd_shot_desc* d) {
 // separable operators (two staggered derivatives and the k^2 term per axis).
 static int setup_conv(qpstd_shot* s, const qpstd_shot_desc* d) {
     HostPlan cx, cz;
-    if (build_conv_plan_host(d->nxx, cx, true) || build_conv_plan_host(d->nzz, cz))
+    if (build_conv_plan_host(d->nxx, cx, kRtX) || build_conv_plan_host(d->nzz, cz, s->blk ? kRtZ : kStockham))
         return fail(QPSTD_ENOTSUP, "no convolution plan for this length");
+    // for the convolution tables and the exact transforms
+    if (s->visco && cx.rt) add_bluestein(cx);
+    if (s->visco && cz.rt && cz.m != cz.n) add_bluestein(cz);
     int rc;
     if ((rc = upload_plan(s, cx, s->pxc))) return rc;
     if ((rc = upload_plan(s, cz, s->pzc))) return rc;
@@ -327,7 +389,7 @@ static int setup_conv(qpstd_shot* s, const qpstd_shot_desc* d) {
         H[j] = k * k / d->nzz;
     }
     put(cz, H, &s->cKz2);
-    CK(cudaMemcpy(base, hc.data(), sizeof(float2) * nc, cudaMemcpyHostToDevice));
+    CK(upload(s, base, hc.data(), sizeof(float2) * nc));
     return QPSTD_OK;
 }
 
@@ -346,7 +408,12 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
     s->d = *d;
     s->arena = arena;
     const int nxx = d->nxx, nzz = d->nzz;
-    const size_t N = (size_t)nxx * nzz;
+    // a line too long for a Stockham plan is refused along z as it always was; along x the
+    // register-to-register passes plan up to 4608 points
+    s->blk = d->method == QPSTD_FUSED && rt_choose(nxx, kRtX) && rt_choose(nzz, kRtZ) && stockham_line(nzz);
+    s->rs = s->blk ? 4 : nzz;
+    s->sb = s->blk ? 4 * (unsigned)nxx : 4;
+    const size_t N = (size_t)nxx * (s->blk ? (nzz + 3) / 4 * 4 : nzz);
     s->N = N;
     s->nx = nxx - 2 * d->pml;
     s->nz = nzz - 2 * d->pml;
@@ -373,7 +440,9 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
             raised[dev] = true;
         }
     }
-    s->nzh = nzz / 2 + 1;
+    // kz columns of the half spectra, an even number (two columns are one aligned access): where
+    // nzz/2 + 1 is odd, the last one repeats the mirrored frequency
+    s->nzh = (nzz / 2 + 2) & ~1;
     cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaStreamCreate"));
 
@@ -390,21 +459,28 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
     s->bbz = dalloc(s, N, &rc);
     s->c1 = dalloc(s, N, &rc);
     s->c2 = dalloc(s, N, &rc);
-    if (!s->div || !s->Lz || !s->bbx || !s->bbz || !s->c1 || !s->c2) return bail(rc);
+    s->io = dalloc(s, (size_t)nxx * nzz, &rc);
+    if (!s->div || !s->Lz || !s->bbx || !s->bbz || !s->c1 || !s->c2 || !s->io) return bail(rc);
+    // the x passes transform the padding of blocked rows beside their points: zeros everywhere
+    for (float* f : {s->div, s->Lz, s->bbx, s->bbz, s->c1, s->c2})
+        if ((e = cudaMemsetAsync(f, 0, sizeof(float) * N, s->stream)) != cudaSuccess) return bail(cuda_fail(e, "memset"));
+    if ((e = cudaMemsetAsync(s->src.st, 0, sizeof(float) * 9 * N, s->stream)) != cudaSuccess) return bail(cuda_fail(e, "memset"));
 
     // models and per-point coefficients (double -> float once)
     {
-        std::vector<float> c1(N), c2(N);
+        const size_t Nu = (size_t)nxx * nzz;
+        std::vector<float> c1(Nu), c2(Nu);
         const double dt = d->dt;
-        for (size_t i = 0; i < N; i++) {
+        for (size_t i = 0; i < Nu; i++) {
             const double vp = d->vp[i];
             c1[i] = (float)((double)d->rho[i] * vp * vp * dt);
             c2[i] = (float)(vp * vp * dt * dt / 12.0);
         }
-        if ((e = cudaMemcpy(s->c1, c1.data(), 4 * N, cudaMemcpyHostToDevice)) != cudaSuccess) return bail(cuda_fail(e, "upload"));
-        if ((e = cudaMemcpy(s->c2, c2.data(), 4 * N, cudaMemcpyHostToDevice)) != cudaSuccess) return bail(cuda_fail(e, "upload"));
-        if ((e = cudaMemcpy(s->bbx, d->bbx, 4 * N, cudaMemcpyHostToDevice)) != cudaSuccess) return bail(cuda_fail(e, "upload"));
-        if ((e = cudaMemcpy(s->bbz, d->bbz, 4 * N, cudaMemcpyHostToDevice)) != cudaSuccess) return bail(cuda_fail(e, "upload"));
+        // c1 in the acoustic x pass, or in z pass C of the low-rank form
+        const bool xc = s->blk && !s->visco;
+        if ((rc = put_field(s, c1.data(), s->c1, xc)) || (rc = put_field(s, c2.data(), s->c2, xc)) ||
+            (rc = put_field(s, d->bbx, s->bbx, s->blk)) || (rc = put_field(s, d->bbz, s->bbz, false)))
+            return bail(rc);
     }
     // 1-D tables
     {
@@ -430,7 +506,7 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
             const double k = wavenumber(j, nzz, d->dz);
             h[o++] = (float)(k * k / nzz);
         }
-        if ((e = cudaMemcpy(base, h.data(), 4 * nt1, cudaMemcpyHostToDevice)) != cudaSuccess) return bail(cuda_fail(e, "upload"));
+        if ((e = upload(s, base, h.data(), 4 * nt1)) != cudaSuccess) return bail(cuda_fail(e, "upload"));
         std::vector<std::complex<double>> H;
         const size_t nc = 2 * (size_t)nxx + 2 * nzz;
         std::vector<float2> hc(nc);
@@ -446,32 +522,57 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
             *cdst[w] = cbase + q;
             for (auto& c : H) hc[q++] = make_float2((float)c.real(), (float)c.imag());
         }
-        if ((e = cudaMemcpy(cbase, hc.data(), sizeof(float2) * nc, cudaMemcpyHostToDevice)) != cudaSuccess) return bail(cuda_fail(e, "upload"));
+        if ((e = upload(s, cbase, hc.data(), sizeof(float2) * nc)) != cudaSuccess) return bail(cuda_fail(e, "upload"));
     }
     // FFT plans and tile shapes of the fused passes (the plain form uses cuFFT)
     if (d->method == QPSTD_FUSED) {
         HostPlan hx, hz;
-        if (build_plan_host(nxx, hx, true) || build_plan_host(nzz, hz))
-            return bail(fail(QPSTD_ENOTSUP, "no FFT plan for this length"));
-        if ((rc = upload_plan(s, hx, s->px))) return bail(rc);
-        if ((rc = upload_plan(s, hz, s->pz))) return bail(rc);
         if ((rc = setup_conv(s, d))) return bail(rc);
+        // exact DFTs: on the convolution plan's entry (its own length, or by Bluestein's
+        // identity) where the passes run one, else a Stockham plan
+        if (s->pxc.rt) {
+            s->px = s->pxc;
+            s->px.blue = 1;
+        } else {
+            if (build_plan_host(nxx, hx)) return bail(fail(QPSTD_ENOTSUP, "no FFT plan for this length"));
+            if ((rc = upload_plan(s, hx, s->px))) return bail(rc);
+        }
+        if (s->pzc.rt) {
+            s->pz = s->pzc;
+            s->pz.blue = s->pz.m != nzz;
+        } else {
+            if (build_plan_host(nzz, hz)) return bail(fail(QPSTD_ENOTSUP, "no FFT plan for this length"));
+            if ((rc = upload_plan(s, hz, s->pz))) return bail(rc);
+        }
         const int pairs_z = (nxx + 1) / 2, pairs_x = (nzz + 1) / 2;
         // acoustic passes: stage the epilogue inputs when they fit beside the lines
         // (z: 5 fields x 2 rows x nzz floats per line; x: up to 9 fields x 2 columns x nxx)
         const size_t stz = (size_t)40 * nzz, stx = xstage_bytes(s->visco, nxx);
-        s->stage_z = ((size_t)8 * s->pzc.m + stz) <= (size_t)QP_SMEM_DYN_MAX;
-        s->stage_x = ((size_t)8 * s->pxc.m + stx) <= (size_t)QP_SMEM_DYN_MAX;
-        s->Lx = choose_L(pairs_x, s->pxc.m, s->pxc.tx, 1, true, s->stage_x ? stx : 0,
+        s->stage_z = !s->pzc.rt && ((size_t)8 * s->pzc.m + stz) <= (size_t)QP_SMEM_DYN_MAX;
+        s->stage_x = !s->pxc.rt && ((size_t)8 * s->pxc.m + stx) <= (size_t)QP_SMEM_DYN_MAX;
+        if (s->pxc.rt) {
+            s->qx = rt_quick(s->pxc.rt, kRtX, pairs_x);
+            s->qs = rt_quick(s->pxc.rt, kRtX, s->nzh);
+        }
+        if (s->pzc.rt) {
+            s->qz = rt_quick(s->pzc.rt, kRtZ, pairs_z);
+            set_quick(s->pz, s->qz);
+            set_quick(s->pzc, s->qz);
+        }
+        s->Lx = s->pxc.rt ? rt_lines(s->pxc.rt, kRtX, s->qx) : choose_L(pairs_x, s->pxc.m, s->pxc.tx, 1, true, s->stage_x ? stx : 0,
                          s->stage_x ? (size_t)QP_SMEM_DYN_MAX : 160 * 1024);
-        s->Lzp = choose_L(pairs_z, s->pzc.m, s->pzc.tx, 1, false, s->stage_z ? stz : 0, 110 * 1024);
+        if (!s->pzc.rt) s->Lzp = choose_L(pairs_z, s->pzc.m, s->pzc.tx, 1, false, s->stage_z ? stz : 0, 110 * 1024);
         if (s->stage_z && (size_t)8 * s->pzc.m + stz > 110 * 1024) s->Lzp = 1;
         // constant-Q: z pass B and the 3-output x-spectral pass hold two line buffers;
         // z pass A uses both the exact and the convolution plan
-        s->Lzv = choose_L(pairs_z, std::max(s->pz.m, s->pzc.m), std::max(s->pz.tx, s->pzc.tx), 2, false);
-        s->Lxs = choose_L(s->nzh, s->px.m, s->px.tx, 1, true);
-        s->Lxs3 = choose_L(s->nzh, s->px.m, s->px.tx, 2, true);
-        const int mmax = std::max(std::max(s->px.m, s->pz.m), std::max(s->pxc.m, s->pzc.m));
+        s->Lzv = s->pzc.rt ? rt_lines(s->pzc.rt, kRtZ, s->qz) : choose_L(pairs_z, std::max(s->pz.m, s->pzc.m), std::max(s->pz.tx, s->pzc.tx), 2, false);
+        if (!s->px.rt) {
+            s->Lxs = choose_L(s->nzh, s->px.m, s->px.tx, 1, true);
+            s->Lxs3 = choose_L(s->nzh, s->px.m, s->px.tx, 2, true);
+        }
+        // (the lines of an rt_list.h entry fit by construction)
+        const int mmax = std::max(std::max(s->px.rt ? 0 : s->px.m, s->pz.rt ? 0 : s->pz.m),
+                                  std::max(s->pxc.rt ? 0 : s->pxc.m, s->pzc.rt ? 0 : s->pzc.m));
         if (16.0 * mmax > 200 * 1024) return bail(fail(QPSTD_ENOTSUP, "line too long for one CTA"));
     }
     if (s->visco && (rc = setup_visco(s, d))) return bail(rc);
@@ -483,18 +584,24 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
     if (s->rtm) {
         s->store = dalloc(s, (size_t)d->snaps * 8 * N, &rc);
         s->obs = dalloc(s, (size_t)d->nt * std::max(d->nr, 1), &rc);
-        s->img = dalloc(s, 4 * (size_t)s->nx * s->nz, &rc);
+        // image and illumination (Kahan pairs): over the whole grid where the register-to-register
+        // passes sum them (acoustic: in the x pass, constant-Q: in z pass C), else the interior
+        s->img_full = s->visco ? s->pz.rt > 0 : s->pxc.rt > 0;
+        s->NI = s->img_full ? N : (size_t)s->nx * s->nz;
+        s->img = dalloc(s, 4 * s->NI, &rc);
         if (!s->store || !s->obs || !s->img) return bail(rc);
-        s->img_c = s->img + (size_t)s->nx * s->nz;
-        s->ssg = s->img_c + (size_t)s->nx * s->nz;
-        s->ssg_c = s->ssg + (size_t)s->nx * s->nz;
+        s->img_c = s->img + s->NI;
+        s->ssg = s->img_c + s->NI;
+        s->ssg_c = s->ssg + s->NI;
     }
     // the receiver lists are grouped by the CTA tiles (x pass: 2*Lx z columns,
     // z pass C: 2*Lzv x rows), so they are built once the tile sizes are final
     if (tune && (rc = autotune(s))) return bail(rc);
     if ((rc = build_receivers(s, d))) return bail(rc);
     s->src.aux_pending = false;
-    if ((e = cudaMemset(s->src.st, 0, sizeof(float) * 9 * N)) != cudaSuccess) return bail(cuda_fail(e, "memset"));
+    if ((e = cudaMemsetAsync(s->src.st, 0, sizeof(float) * 9 * N, s->stream)) != cudaSuccess) return bail(cuda_fail(e, "memset"));
+    // the uploads have left the host buffers and later work may come on any stream
+    if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) return bail(cuda_fail(e, "create"));
     *out = s;
     return QPSTD_OK;
 }
@@ -519,7 +626,13 @@ extern "C" int qpstd_shot_destroy(qpstd_shot* s) {
 
 extern "C" int qpstd_shot_set_state(qpstd_shot* s, const float* state) {
     if (!s || !state) return fail(QPSTD_EINVAL, "null argument");
-    CK(cudaMemcpyAsync(s->src.st, state, sizeof(float) * 8 * s->N, cudaMemcpyHostToDevice, s->stream));
+    if (!s->blk) {
+        CK(upload(s, s->src.st, state, sizeof(float) * 8 * s->N));
+    } else {
+        const size_t n = (size_t)s->d.nxx * s->d.nzz;
+        for (int k = 0; k < 8; k++)
+            if (const int rc = put_field(s, state + k * n, s->src.st + k * s->N, state_blocked(s, k))) return rc;
+    }
     CK(cudaStreamSynchronize(s->stream));
     s->src.aux_pending = false;
     return QPSTD_OK;
@@ -527,7 +640,13 @@ extern "C" int qpstd_shot_set_state(qpstd_shot* s, const float* state) {
 
 extern "C" int qpstd_shot_get_state(qpstd_shot* s, float* state) {
     if (!s || !state) return fail(QPSTD_EINVAL, "null argument");
-    CK(cudaMemcpyAsync(state, s->src.st, sizeof(float) * 8 * s->N, cudaMemcpyDeviceToHost, s->stream));
+    if (!s->blk) {
+        CK(cudaMemcpyAsync(state, s->src.st, sizeof(float) * 8 * s->N, cudaMemcpyDeviceToHost, s->stream));
+    } else {
+        const size_t n = (size_t)s->d.nxx * s->d.nzz;
+        for (int k = 0; k < 8; k++)
+            if (const int rc = get_window(s, s->src.st + k * s->N, state_blocked(s, k), s->d.nxx, s->d.nzz, 0, 0, state + k * n)) return rc;
+    }
     CK(cudaStreamSynchronize(s->stream));
     return QPSTD_OK;
 }
@@ -590,6 +709,9 @@ static AcZArgs zargs(qpstd_shot* s, Wave& w, int do_v, int do_div) {
     a.dt = s->d.dt;
     a.do_v = do_v;
     a.do_div = do_div;
+    a.rs = s->rs;
+    a.sb = s->sb;
+    a.rz = s->d.nzz;
     a.stage = s->stage_z ? 1 : 0;
     return a;
 }
@@ -602,6 +724,7 @@ static AcXArgs xargs(qpstd_shot* s, Wave& w, int do_p, int do_v, int do_dx) {
     a.L = s->Lx;
     a.pml = s->d.pml;
     a.pl = s->pxc;
+    set_quick(a.pl, s->qx);
     a.HxP = s->cHxP;
     a.HxM = s->cHxM;
     a.kx2 = s->cKx2;
@@ -625,6 +748,8 @@ static AcXArgs xargs(qpstd_shot* s, Wave& w, int do_p, int do_v, int do_dx) {
     a.do_dx = do_dx;
     a.xs = -1;
     a.zs = -1;
+    a.rs = s->rs;
+    a.sb = s->sb;
     a.stage = s->stage_x ? 1 : 0;
     return a;
 }
@@ -683,6 +808,16 @@ static bool filter_is_ka(qpstd_shot* s, float eta, int t) {
     return t <= lo;
 }
 
+// Strides of the fields and of the half spectra: column pairs of a blocked shot's spectra are
+// contiguous along x.
+template <class A> static void set_strides(const qpstd_shot* s, A& a) {
+    a.rs = s->rs;
+    a.sb = s->sb;
+    a.rz = s->d.nzz;
+    a.srs = s->blk ? 2 : s->nzh;
+    a.ssb = s->blk ? 2 * (unsigned)s->d.nxx : 2;
+}
+
 // One constant-Q step of wavefield w (seven launches, see vz_kernels.cu).
 // src: amplitude at the source this step; t_filter / eta: time index and
 // stabilisation of the Q-RTM aux filter; last: skip the next step's Dx;
@@ -701,6 +836,7 @@ static void vz_step(qpstd_shot* s, Wave& w, float src, int t_filter, float eta, 
         a.aux_spec = w.aux_pending ? w.aux_spec : nullptr;
         a.aux = w.aux(N); a.vz = w.vz(N); a.psi_vz = w.fivzz(N); a.Dx = w.Dx(N);
         a.div = s->div; a.G = s->spec[0];
+        set_strides(s, a);
         ProfScope ps(s, QPSTD_K_ZPASS);
         launch_vz_passA(a, st);
         w.aux_pending = false;
@@ -708,10 +844,24 @@ static void vz_step(qpstd_shot* s, Wave& w, float src, int t_filter, float eta, 
     VxsArgs xs{};
     xs.nxx = nxx; xs.nzz = nzz; xs.nzh = nzh; xs.pl = s->px; xs.kx2 = s->kxsq; xs.kz2 = s->kzsq; xs.norm = norm;
     xs.plc = s->pxc;
+    XconvArgs xc{};
+    xc.nxx = nxx; xc.nzh = nzh; xc.pl = s->pxc;
+    xc.srs = xs.srs = s->blk ? 2 : nzh;
+    xc.ssb = xs.ssb = s->blk ? 2 * (unsigned)nxx : 2;
+    set_quick(xc.pl, s->qs);
     // modes 0 and 1 (stationary symbols): per-kz convolution tables when built;
     // launches on exact DFTs are timed as their own kind
     auto xspec = [&](VxsArgs& a) {
-        if (s->xconv && a.mode != 2) {
+        if (s->pxc.rt && a.mode != 2) {
+            xc.nout = a.mode == 0 ? 3 : 1;
+            xc.in = a.in;
+            xc.out = a.out0;
+            xc.out_step = (size_t)nxx * nzh;  // out0 .. out2 are consecutive
+            xc.tab = s->xtab[a.mode == 0 ? 0 : 3];
+            xc.tab_step = (size_t)nzh * (s->pxc.m / 2 + 1);
+            ProfScope ps(s, QPSTD_K_XSPEC);
+            launch_rt_xconv(xc, st);
+        } else if (s->xconv && a.mode != 2) {
             a.tab0 = s->xtab[a.mode == 0 ? 0 : 3];
             a.tab1 = s->xtab[1];
             a.tab2 = s->xtab[2];
@@ -725,16 +875,27 @@ static void vz_step(qpstd_shot* s, Wave& w, float src, int t_filter, float eta, 
     const bool lowrank = s->lr_row > 0;
     if (lowrank) {
         // low-rank form: total <- W{div} = sum_b c_b Re F^-1[Vt_b F div] / N
-        LrxArgs x{};
-        x.nxx = nxx; x.nzh = nzh; x.L = s->Llr; x.row = s->lr_row; x.plc = s->pxc;
-        x.in = s->spec[0]; x.out = s->lr_Q; x.tab = s->lr_tab;
-        {
+        if (s->pxc.rt) {
+            xc.nout = s->lr_row;
+            xc.in = s->spec[0];
+            xc.out = s->lr_Q;
+            xc.out_step = (size_t)nxx * nzh;
+            xc.tab = s->lr_tab;
+            xc.tab_step = (size_t)nzh * (s->pxc.m / 2 + 1);
+            ProfScope ps(s, QPSTD_K_XSPEC);
+            launch_rt_xconv(xc, st);
+        } else {
+            LrxArgs x{};
+            x.nxx = nxx; x.nzh = nzh; x.L = s->Llr; x.row = s->lr_row; x.plc = s->pxc;
+            x.in = s->spec[0]; x.out = s->lr_Q; x.tab = s->lr_tab;
             ProfScope ps(s, QPSTD_K_XSPEC);
             launch_lr_xconv(x, st);
         }
         LrsArgs z{};
         z.nxx = nxx; z.nzz = nzz; z.nzh = nzh; z.L = s->Llrz; z.row = s->lr_row; z.pl = s->pz;
         z.Q = s->lr_Q; z.c = s->lr_c; z.psc = s->total;
+        z.npts = N;
+        set_strides(s, z);
         ProfScope ps(s, QPSTD_K_ZPASS);
         launch_lr_zsum(z, st);
     } else {
@@ -750,6 +911,7 @@ static void vz_step(qpstd_shot* s, Wave& w, float src, int t_filter, float eta, 
             a.Y2 = s->spec[1]; a.Y3 = s->spec[2]; a.Y4 = s->spec[3];
             a.div = s->div; a.y1 = s->y1; a.y2 = s->y2; a.y3c = s->y3c; a.y4c = s->y4c;
             a.total = s->total; a.T = s->spec[0];
+            set_strides(s, a);
             ProfScope ps(s, QPSTD_K_ZPASS);
             launch_vz_passB(a, st);
         }
@@ -773,8 +935,9 @@ static void vz_step(qpstd_shot* s, Wave& w, float src, int t_filter, float eta, 
         a.gather_row = gather_row; a.obs_row = obs_row;
         if (ssg_on) { a.ssg = s->ssg; a.ssg_c = s->ssg_c; }
         if (image) { a.img = s->img; a.img_c = s->img_c; a.ps = s->src.p(N); }
-        a.P = s->spec[2]; a.HzP = s->HzP; a.h_az = s->h_az; a.h_bz = s->h_bz; a.bbz = s->bbz;
+        a.P = s->spec[2]; a.HzP = s->pz.rt ? s->cHzP : s->HzP; a.h_az = s->h_az; a.h_bz = s->h_bz; a.bbz = s->bbz;
         a.vz = w.vz(N); a.psi_pz = w.fipz(N); a.dt = s->d.dt;
+        set_strides(s, a);
         ProfScope ps(s, QPSTD_K_ZPASS);
         launch_vz_passC(a, st);
     }
@@ -793,7 +956,7 @@ static void vz_step(qpstd_shot* s, Wave& w, float src, int t_filter, float eta, 
         } else {
             a.mode = 1;
         }
-        if (a.mode == 2 && s->xconv) a.L = s->Lxs_exact;
+        if (a.mode == 2 && s->xconv && !s->pxc.rt) a.L = s->Lxs_exact;
         xspec(a);
         w.aux_pending = true;
     }
@@ -802,11 +965,19 @@ static void vz_step(qpstd_shot* s, Wave& w, float src, int t_filter, float eta, 
 // Turn a pending aux spectrum back into the real aux field.
 static void vz_finish(qpstd_shot* s, Wave& w) {
     if (!w.aux_pending) return;
-    VzArgsI a{};
-    a.nxx = s->d.nxx; a.nzz = s->d.nzz; a.nzh = s->nzh; a.L = s->Lzv; a.pl = s->pz;
-    a.spec = w.aux_spec; a.out = w.aux(s->N);
     ProfScope ps(s, QPSTD_K_ZPASS);
-    launch_vz_zinv(a, s->stream);
+    if (s->pz.rt) {
+        LrsArgs z{};
+        z.nxx = s->d.nxx; z.nzz = s->d.nzz; z.nzh = s->nzh; z.row = 1; z.pl = s->pz;
+        z.Q = w.aux_spec; z.psc = w.aux(s->N);
+        set_strides(s, z);
+        launch_lr_zsum(z, s->stream);
+    } else {
+        VzArgsI a{};
+        a.nxx = s->d.nxx; a.nzz = s->d.nzz; a.nzh = s->nzh; a.L = s->Lzv; a.pl = s->pz;
+        a.spec = w.aux_spec; a.out = w.aux(s->N);
+        launch_vz_zinv(a, s->stream);
+    }
     w.aux_pending = false;
 }
 
@@ -914,15 +1085,17 @@ static std::vector<Knob> shot_knobs(qpstd_shot* s) {
     if (s->visco) {
         const int mz = std::max(s->pz.m, s->pzc.m), tz = std::max(s->pz.tx, s->pzc.tx);
         const FFTPlanDev& pxs = s->xconv ? s->pxc : s->px;
-        knobs.push_back({&s->Lzv, false, tz, (size_t)16 * mz, vzb});  // z passes A-C share L
-        knobs.push_back({&s->Lxs3, true, pxs.tx, (size_t)16 * pxs.m, vzb});
-        knobs.push_back({&s->Lxs, true, pxs.tx, (size_t)8 * pxs.m, vzb});
-        if (s->xconv && s->d.kind == QPSTD_QRTM)
+        if (!s->pz.rt) knobs.push_back({&s->Lzv, false, tz, (size_t)16 * mz, vzb});  // z passes A-C share L
+        if (!pxs.rt) {
+            knobs.push_back({&s->Lxs3, true, pxs.tx, (size_t)16 * pxs.m, vzb});
+            knobs.push_back({&s->Lxs, true, pxs.tx, (size_t)8 * pxs.m, vzb});
+        }
+        if (s->xconv && s->d.kind == QPSTD_QRTM && !s->pxc.rt)
             knobs.push_back({&s->Lxs_exact, true, s->px.tx, (size_t)8 * s->px.m, vzb});
-    } else {
+    } else if (!s->pzc.rt) {
         knobs.push_back({&s->Lzp, false, s->pzc.tx, (size_t)8 * s->pzc.m, acb, &s->stage_z, stz});
     }
-    knobs.push_back({&s->Lx, true, s->pxc.tx, (size_t)8 * s->pxc.m, acb, &s->stage_x, stx});
+    if (!s->pxc.rt) knobs.push_back({&s->Lx, true, s->pxc.tx, (size_t)8 * s->pxc.m, acb, &s->stage_x, stx});
     return knobs;
 }
 
@@ -963,6 +1136,7 @@ static int autotune(qpstd_shot* s) {
     const char* env = getenv("QPSTD_AUTOTUNE");
     if (s->d.method != QPSTD_FUSED || (env && env[0] == '0')) return QPSTD_OK;
     std::vector<Knob> knobs = shot_knobs(s);
+    if (knobs.empty()) return QPSTD_OK;
     // cached per shape: L * 2 + staging
     const std::vector<int> key = {s->d.kind, s->d.nxx, s->d.nzz};
     {
@@ -1042,14 +1216,19 @@ extern "C" long long qpstd_shot_bytes(const qpstd_shot_desc* d) {
     if (!d || d->nxx < 1 || d->nzz < 1 || d->nt < 1) return -1;
     const bool visco = d->kind == QPSTD_VAPS || d->kind == QPSTD_QRTM;
     const bool rtm = d->kind == QPSTD_ARTM || d->kind == QPSTD_QRTM;
-    const double N = (double)d->nxx * d->nzz, nzh = d->nzz / 2 + 1, NS = d->nxx * nzh;
-    const double nr = std::max(d->nr, 1), nx = d->nxx - 2 * d->pml, nz = d->nzz - 2 * d->pml;
     const bool fused = d->method != QPSTD_PLAIN;
+    const int ix = rt_choose(d->nxx, kRtX), iz = ix && stockham_line(d->nzz) ? rt_choose(d->nzz, kRtZ) : 0;
+    const bool blk = fused && iz;
+    const double Nu = (double)d->nxx * d->nzz, N = blk ? (double)d->nxx * ((d->nzz + 3) / 4 * 4) : Nu;
+    const double nzh = (d->nzz / 2 + 2) & ~1, NS = d->nxx * nzh;
+    const double nr = std::max(d->nr, 1), nx = d->nxx - 2 * d->pml, nz = d->nzz - 2 * d->pml;
     HostPlan cx, cz, ex, ez;
-    if (fused && (build_conv_plan_host(d->nxx, cx, true) || build_conv_plan_host(d->nzz, cz) ||
-                  build_plan_host(d->nxx, ex, true) || build_plan_host(d->nzz, ez)))
+    if (ix) cx.m = ex.m = rt_length(ix, kRtX);
+    if (iz) cz.m = ez.m = rt_length(iz, kRtZ);
+    if (fused && ((!ix && (build_conv_plan_host(d->nxx, cx) || build_plan_host(d->nxx, ex))) ||
+                  (!iz && (build_conv_plan_host(d->nzz, cz) || build_plan_host(d->nzz, ez)))))
         return -1;  // no fused plan for these lengths
-    double f = (rtm ? 18.0 : 9.0) * N + 6.0 * N;                       // wavefields; div, Lz, bbx, bbz, c1, c2
+    double f = (rtm ? 18.0 : 9.0) * N + 6.0 * N + Nu;                  // wavefields; div, Lz, bbx, bbz, c1, c2; conversions
     if (fused) {
         f += 2.0 * (cx.m + cz.m) + 6.0 * (cx.m + cz.m);                // convolution plans and multipliers
         f += 2.0 * (2.0 * ex.m + d->nxx) + 2.0 * (2.0 * ez.m + d->nzz);  // exact plans (twiddles, chirp, bhat)
@@ -1057,10 +1236,10 @@ extern "C" long long qpstd_shot_bytes(const qpstd_shot_desc* d) {
     f += 16.0 * (d->nxx + d->nzz);                                     // CPML profiles, squared wavenumbers
     if (visco) {
         f += 8.0 * N + 2.0 * NS * (rtm ? 6 : 5) + 4.0 * (d->nxx + d->nzz);
-        if (fused && ex.blue) f += 4.0 * nzh * (cx.m / 2 + 1);         // per-kz convolution tables
+        if (fused && (ix || ex.blue)) f += 4.0 * nzh * (cx.m / 2 + 1);         // per-kz convolution tables
     }
     f += (double)d->nt * nr;                                           // gather
-    if (rtm) f += (double)d->snaps * 8.0 * N + (double)d->nt * nr + 4.0 * nx * nz;
+    if (rtm) f += (double)d->snaps * 8.0 * N + (double)d->nt * nr + 4.0 * (fused && ix ? N : nx * nz);
     if (d->method == QPSTD_PLAIN) f += 20.0 * N;
     return (long long)(4.0 * f) + 32 * 256 + (1ll << 20);
 }
@@ -1180,33 +1359,36 @@ extern "C" int qpstd_shot_set_lowrank(qpstd_shot* s, int row, int col, const flo
     if (row < 1 || col < 1 || row > 16 || col > 16 || !U || !V || !A)
         return fail(QPSTD_EINVAL, "low-rank factors: 1 <= row, col <= 16 and U, V, A non-null");
     if (s->lr_row) return fail(QPSTD_EINVAL, "the shot already runs the low-rank form");
-    const int nxx = s->d.nxx, nzz = s->d.nzz, nzh = s->nzh, nxh = nxx / 2 + 1;
-    const size_t N = s->N;
+    const int nxx = s->d.nxx, nzz = s->d.nzz, nzh = s->nzh, nxh = nxx / 2 + 1, nvh = nzz / 2 + 1;
+    const size_t N = s->N, Nu = (size_t)nxx * nzz;
     const int mc = s->pxc.m, mh = mc / 2 + 1;
     int rc = QPSTD_OK;
     float* c = dalloc(s, (size_t)row * N, &rc);
     float* tab = c ? dalloc(s, (size_t)row * nzh * mh, &rc) : nullptr;
     float* Q = tab ? dalloc(s, (size_t)row * 2 * nxx * nzh, &rc) : nullptr;
-    float* Vd = Q ? dalloc(s, (size_t)row * nxh * nzh, &rc) : nullptr;
+    float* Vd = Q ? dalloc(s, (size_t)row * nxh * nvh, &rc) : nullptr;
     if (!Vd) return rc;
-    std::vector<float> hc((size_t)row * N);
-    for (size_t x = 0; x < N; x++)
+    std::vector<float> hc((size_t)row * Nu);
+    for (size_t x = 0; x < Nu; x++)
         for (int b = 0; b < row; b++) {
             double acc = 0.0;
             for (int a = 0; a < col; a++) acc += (double)U[x * col + a] * A[(size_t)a * row + b];
-            hc[(size_t)b * N + x] = (float)acc;
+            hc[(size_t)b * Nu + x] = (float)acc;
         }
-    CK(cudaMemcpy(c, hc.data(), sizeof(float) * hc.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(Vd, V, sizeof(float) * (size_t)row * nxh * nzh, cudaMemcpyHostToDevice));
+    CK(cudaMemsetAsync(c, 0, sizeof(float) * (size_t)row * N, s->stream));
+    for (int b = 0; b < row; b++)
+        if ((rc = put_field(s, hc.data() + (size_t)b * Nu, c + (size_t)b * N, false))) return rc;
+    CK(cudaMemsetAsync(Q, 0, sizeof(float) * (size_t)row * 2 * nxx * nzh, s->stream));
+    CK(upload(s, Vd, V, sizeof(float) * (size_t)row * nxh * nvh));
     VtabArgs a{};
     a.nxx = nxx; a.nzz = nzz; a.nzh = nzh;
     a.pl = s->px; a.plc = s->pxc; a.kx2 = s->kxsq; a.kz2 = s->kzsq;
     a.norm = (float)(1.0 / ((double)nxx * nzz));
-    a.L = choose_L(nzh, std::max(s->px.m, mc), std::max(s->px.tx, s->pxc.tx), 1, false);
+    if (!s->pxc.rt) a.L = choose_L(nzh, std::max(s->px.m, mc), std::max(s->px.tx, s->pxc.tx), 1, false);
     a.sym = 4;
     a.nxh = nxh;
     for (int b = 0; b < row; b++) {
-        a.V = Vd + (size_t)b * nxh * nzh;
+        a.V = Vd + (size_t)b * nxh * nvh;
         a.out = tab + (size_t)b * nzh * mh;
         launch_vz_convtab(a, s->stream);
     }
@@ -1216,8 +1398,8 @@ extern "C" int qpstd_shot_set_lowrank(qpstd_shot* s, int row, int col, const flo
     s->lr_c = c;
     s->lr_tab = tab;
     s->lr_Q = reinterpret_cast<float2*>(Q);
-    s->Llr = choose_L(nzh, mc, s->pxc.tx, 2, true);
-    s->Llrz = choose_L((nxx + 1) / 2, s->pz.m, s->pz.tx, 2, false);
+    if (!s->pxc.rt) s->Llr = choose_L(nzh, mc, s->pxc.tx, 2, true);
+    if (!s->pz.rt) s->Llrz = choose_L((nxx + 1) / 2, s->pz.m, s->pz.tx, 2, false);
     s->lr_row = row;
     return QPSTD_OK;
 }
@@ -1301,7 +1483,7 @@ extern "C" int qpstd_shot_set_obs(qpstd_shot* s, const float* obs) {
 // the actions of its shots, so their work overlaps on the device.
 int rtm_begin(qpstd_shot* s) {
     if (!s || !s->rtm) return fail(QPSTD_EINVAL, "not an RTM shot");
-    const size_t N = s->N, NI = (size_t)s->nx * s->nz;
+    const size_t N = s->N, NI = s->NI;
     cudaStream_t st = s->stream;
     s->launches = 0;
     s->fwd_steps = 0;
@@ -1341,7 +1523,7 @@ int rtm_action(qpstd_shot* s) {
         if (r.rv.capo() == 0) {
             // checkpoint 0 also holds the first source sample (acsglw.cu:493-500)
             ProfScope ps(s, QPSTD_K_OTHER);
-            add_point_kernel<<<1, 1, 0, st>>>(slot + (size_t)s->d.xsg * s->d.nzz + s->d.zsg,
+            add_point_kernel<<<1, 1, 0, st>>>(slot + field_at(s, s->d.xsg, s->d.zsg),
                                               (float)((double)s->rik[0] * 1000.0 * s->d.dt));
         }
     } else if (act == RV_ADVANCE) {
@@ -1389,8 +1571,14 @@ extern "C" int qpstd_shot_rtm_device(qpstd_shot* s) {
 extern "C" int qpstd_shot_get_image(qpstd_shot* s, float* img, float* ssg) {
     if (!s || !s->rtm) return fail(QPSTD_EINVAL, "not an RTM shot");
     const size_t NI = (size_t)s->nx * s->nz;
-    if (img) CK(cudaMemcpyAsync(img, s->img, sizeof(float) * NI, cudaMemcpyDeviceToHost, s->stream));
-    if (ssg) CK(cudaMemcpyAsync(ssg, s->ssg, sizeof(float) * NI, cudaMemcpyDeviceToHost, s->stream));
+    int rc;
+    if (s->img_full) {
+        if (img && (rc = get_window(s, s->img, s->blk && !s->visco, s->nx, s->nz, s->d.pml, s->d.pml, img))) return rc;
+        if (ssg && (rc = get_window(s, s->ssg, s->blk && !s->visco, s->nx, s->nz, s->d.pml, s->d.pml, ssg))) return rc;
+    } else {
+        if (img) CK(cudaMemcpyAsync(img, s->img, sizeof(float) * NI, cudaMemcpyDeviceToHost, s->stream));
+        if (ssg) CK(cudaMemcpyAsync(ssg, s->ssg, sizeof(float) * NI, cudaMemcpyDeviceToHost, s->stream));
+    }
     CK(cudaStreamSynchronize(s->stream));
     return QPSTD_OK;
 }

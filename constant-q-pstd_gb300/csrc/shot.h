@@ -78,6 +78,13 @@ struct qpstd_shot {
     const float2 *cHxM = nullptr, *cHxP = nullptr, *cKx2 = nullptr;  // convolution multipliers
     const float2 *cHzM = nullptr, *cHzP = nullptr, *cKz2 = nullptr;
     int Lx = 1, Lzp = 1, ntile_x = 0;
+    int qx = 0, qs = 0, qz = 0;             // quick form of the x pass / x-spectral / z passes (rt_list.h)
+    // layout of the device fields (rt_z.cuh): blocked or row by row, and their strides; N counts
+    // the padding; io: nxx * nzz floats for the conversions from and to the caller's layout
+    bool blk = false, img_full = false;
+    unsigned rs = 0, sb = 0;
+    size_t NI = 0;                          // points of img, img_c, ssg, ssg_c
+    float* io = nullptr;
     bool stage_x = false, stage_z = false;  // acoustic passes stage epilogue inputs
     int* rec_off = nullptr;
     qp::RecEntry* rec = nullptr;

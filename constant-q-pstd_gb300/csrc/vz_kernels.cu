@@ -1,6 +1,6 @@
 // vz_kernels.cu -- launchers of the constant-Q pass kernels (vz_kernels.cuh).
 #include "vz_kernels.cuh"
-#include "xplans.cuh"
+#include "rt.cuh"
 
 namespace qp {
 
@@ -15,6 +15,10 @@ using ZPlans = PlanList<CtFFT<11, 10, 6>, CtFFT<5, 5, 8>>;
 
 
 void launch_vz_passA(const VzArgsA& a, cudaStream_t s) {
+    if (a.pl.rt) {
+        rtz_any(a.pl.quick, [&](const RtzGroup& g) { return g.passA(a, s); });
+        return;
+    }
     const dim3 blk(max(a.pl.tx, a.plc.tx), a.L);
     const size_t sm = lsm(a.L, max(a.pl.m, a.plc.m), 1);
     const bool r12 = plan_max_radix(a.pl) <= 12 && plan_max_radix(a.plc) <= 12;
@@ -24,16 +28,21 @@ void launch_vz_passA(const VzArgsA& a, cudaStream_t s) {
 #undef L_
 }
 void launch_vz_xspec(const VxsArgs& a, cudaStream_t s) {
+    if (a.pl.rt) {
+        rt_any(false, [&](const RtGroup& g) { return g.xexact(a, s); });
+        return;
+    }
     const int grid = (a.nzh + a.L - 1) / a.L;
     const size_t sm = lsm(a.L, a.pl.m, a.mode == 0 ? 2 : 1);
-    if (xplan_launch_xspec(a, s, dim3(grid), dim3(a.pl.tx, a.L), sm)) return;  // a compiled long plan
     if (plan_max_radix(a.pl) <= 12) vz_xspec_kernel<RtFFT<12>><<<grid, dim3(a.pl.tx, a.L), sm, s>>>(a);
     else vz_xspec_kernel<RtFFT<16>><<<grid, dim3(a.pl.tx, a.L), sm, s>>>(a);
+}
+void launch_rt_xconv(const XconvArgs& a, cudaStream_t s) {
+    rt_any(a.pl.quick, [&](const RtGroup& g) { return g.xconv(a, s); });
 }
 void launch_vz_xspec_conv(const VxsArgs& a, cudaStream_t s) {
     const int grid = (a.nzh + a.L - 1) / a.L;
     const dim3 blk(a.plc.tx, a.L);
-    if (xplan_launch_xspec_conv(a, s, dim3(grid), blk, lsm(a.L, a.plc.m, a.mode == 0 ? 2 : 1))) return;
     const bool r12 = plan_max_radix(a.plc) <= 12;
     if (a.mode == 0 && r12) vz_xspec_conv_kernel<3, RtFFT<12>><<<grid, blk, lsm(a.L, a.plc.m, 2), s>>>(a);
     else if (a.mode == 0) vz_xspec_conv_kernel<3, RtFFT<16>><<<grid, blk, lsm(a.L, a.plc.m, 2), s>>>(a);
@@ -41,21 +50,27 @@ void launch_vz_xspec_conv(const VxsArgs& a, cudaStream_t s) {
     else vz_xspec_conv_kernel<1, RtFFT<16>><<<grid, blk, lsm(a.L, a.plc.m, 1), s>>>(a);
 }
 void launch_vz_convtab(const VtabArgs& a, cudaStream_t s) {
+    if (a.plc.rt) {
+        rt_any(false, [&](const RtGroup& g) { return g.convtab(a, s); });
+        return;
+    }
     const int grid = (a.nzh + a.L - 1) / a.L;
     const dim3 blk(max(a.pl.tx, a.plc.tx), a.L);
     const size_t sm = lsm(a.L, max(a.pl.m, a.plc.m), 1);
-    if (xplan_launch_convtab(a, s, dim3(grid), blk, sm)) return;  // a compiled long plan
     vz_convtab_kernel<RtFFT<16>><<<grid, blk, sm, s>>>(a);
 }
 void launch_lr_xconv(const LrxArgs& a, cudaStream_t s) {
     const int grid = (a.nzh + a.L - 1) / a.L;
     const dim3 blk(a.plc.tx, a.L);
     const size_t sm = lsm(a.L, a.plc.m, 2);
-    if (xplan_launch_lr_xconv(a, s, dim3(grid), blk, sm)) return;  // a compiled long plan
     if (plan_max_radix(a.plc) <= 12) lr_xconv_kernel<RtFFT<12>><<<grid, blk, sm, s>>>(a);
     else lr_xconv_kernel<RtFFT<16>><<<grid, blk, sm, s>>>(a);
 }
 void launch_lr_zsum(const LrsArgs& a, cudaStream_t s) {
+    if (a.pl.rt) {
+        rtz_any(a.pl.quick, [&](const RtzGroup& g) { return g.zsum(a, s); });
+        return;
+    }
     const dim3 blk(a.pl.tx, a.L);
     const size_t sm = lsm(a.L, a.pl.m, 2);
 #define L_(FPT)                                                                         \
@@ -66,6 +81,10 @@ void launch_lr_zsum(const LrsArgs& a, cudaStream_t s) {
 }
 
 void launch_vz_passB(const VzArgsB& a, cudaStream_t s) {
+    if (a.pl.rt) {
+        rtz_any(a.pl.quick, [&](const RtzGroup& g) { return g.passB(a, s); });
+        return;
+    }
     const dim3 blk(a.pl.tx, a.L);
     const size_t sm = lsm(a.L, a.pl.m, 2);
 #define L_(FPT) vz_passB_kernel<FPT><<<zgrid(a.nxx, a.L), blk, sm, s>>>(a)
@@ -73,6 +92,10 @@ void launch_vz_passB(const VzArgsB& a, cudaStream_t s) {
 #undef L_
 }
 void launch_vz_passC(const VzArgsC& a, cudaStream_t s) {
+    if (a.pl.rt) {
+        rtz_any(a.pl.quick, [&](const RtzGroup& g) { return g.passC(a, s); });
+        return;
+    }
     const dim3 blk(a.pl.tx, a.L);
     const size_t sm = lsm(a.L, a.pl.m, 1);
 #define L_(FPT) vz_passC_kernel<FPT><<<zgrid(a.nxx, a.L), blk, sm, s>>>(a)

@@ -137,19 +137,6 @@ __global__ void __maxnreg__(FP::kMaxRadix <= 12 ? QP_R12_REGS : QP_PASS_REGS) vz
 
 // ---- x-spectral pass ----------------------------------------------------------
 // L kz columns per CTA (L a power of two); line c = column kz0 + c.
-__device__ __forceinline__ float spec_symbol(const VxsArgs& a, int j, float k2) {
-    if (a.mode == 0) {
-        if (j == 1) return k2;
-        const float k32 = exp2f(log2f(k2) * (1.f / 32.f));
-        return (j == 0) ? k32 : k2 * k32;
-    }
-    const float ka = exp2f(0.505f * log2f(k2));
-    if (a.mode == 1) return ka;
-    const float num = 2.f * a.eta6 * ka * (1.f + a.tao * a.dt * ka);
-    const float den = expf(-a.tao * a.tt * ka) + a.eta6 * expf(a.tao * a.dt * ka);
-    return ka - num / den;
-}
-
 // FP: transform policy of the exact plan (Bluestein plans included).
 template <class FP>
 __global__ void __maxnreg__(FP::kMaxRadix <= 12 ? QP_PASS_REGS : QP_EXACT_REGS) vz_xspec_kernel(VxsArgs a) {
@@ -287,11 +274,7 @@ __global__ void __launch_bounds__(768, 1) vz_convtab_kernel(VtabArgs a) {
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
         const double k2 = (double)a.kx2[k] + kzsq;
         double s;
-        if (a.sym == 4) s = a.V[(size_t)((k < a.nxh) ? k : n - k) * a.nzh + (valid ? kz : 0)];
-        else if (a.sym == 1) s = k2;
-        else if (a.sym == 0) s = pow(k2, 1.0 / 32.0);
-        else if (a.sym == 2) s = pow(k2, 33.0 / 32.0);
-        else s = pow(k2, 0.505);
+        s = tab_symbol(a, k, valid ? kz : 0, k2);
         line[k] = make_float2((float)s, 0.f);
     }
     __syncthreads();
