@@ -11,6 +11,7 @@
 #include "host_setup.h"
 
 #include <initializer_list>
+#include <memory>
 
 #include "rt_list.h"
 
@@ -192,36 +193,95 @@ static bool factor_direct(int n, std::vector<int>& rad) {
     return n / rmin <= QP_MAXTHREADS;
 }
 
-// Host Stockham in double (same recurrence as the device engine).
-static void host_fft(std::vector<std::complex<double>>& x, const std::vector<int>& rad, int sgn) {
-    const int n = (int)x.size();
-    std::vector<std::complex<double>> y(n);
-    std::vector<std::complex<double>>*src = &x, *dst = &y;
-    int ns = 1;
-    for (int r : rad) {
-        const int nb = n / r;
-        for (int j = 0; j < nb; j++) {
-            const int k = j % ns;
-            std::complex<double> v[32], o[32];
-            for (int q = 0; q < r; q++) {
-                const double ang = sgn * 2.0 * M_PI * (double)(q * k) / (double)(ns * r);
-                v[q] = (*src)[j + q * nb] * std::complex<double>(std::cos(ang), std::sin(ang));
-            }
-            for (int q = 0; q < r; q++) {
-                std::complex<double> acc = 0;
-                for (int u = 0; u < r; u++) {
-                    const double ang = sgn * 2.0 * M_PI * (double)((u * q) % r) / (double)r;
-                    acc += v[u] * std::complex<double>(std::cos(ang), std::sin(ang));
-                }
-                o[q] = acc;
-            }
-            const int base = (j - k) * r + k;
-            for (int q = 0; q < r; q++) (*dst)[base + q * ns] = o[q];
-        }
-        std::swap(src, dst);
-        ns *= r;
+// ---- FP64 transforms of the table setup ------------------------------------------
+// Stockham passes of small radices on a table of roots: the multipliers of a shot take about
+// twenty transforms of the convolution lengths, which evaluated root by root (and the sums over
+// the window's own DFT term by term) were most of a shot's creation.
+namespace {
+struct Cd {
+    double x, y;
+};
+inline Cd mul(Cd a, Cd b) { return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x}; }
+
+struct HostFFT {
+    int n;
+    std::vector<int> rad;
+    std::vector<Cd> w, tmp;  // w[k] = e^{-2 pi i k / n}
+    explicit HostFFT(int n_) : n(n_), w(n_), tmp(n_) {
+        int v = n;
+        for (int f : {4, 3, 5, 7, 11, 13, 2})
+            for (; v % f == 0; v /= f) rad.push_back(f);
+        for (int k = 0; k < n; k++) w[k] = {std::cos(2.0 * M_PI * k / n), -std::sin(2.0 * M_PI * k / n)};
     }
-    if (src != &x) x = *src;
+    // sgn -1: forward, +1: inverse, unnormalised
+    void run(std::vector<Cd>& x, int sgn) {
+        Cd *src = x.data(), *dst = tmp.data();
+        int ns = 1;
+        for (int r : rad) {
+            const int nb = n / r, step = n / (ns * r), rs = n / r;
+            for (int j = 0; j < nb; j++) {
+                const int k = j % ns;
+                Cd v[13];
+                v[0] = src[j];
+                for (int q = 1; q < r; q++) {
+                    Cd t = w[q * k * step];
+                    if (sgn > 0) t.y = -t.y;
+                    v[q] = mul(src[j + q * nb], t);
+                }
+                Cd* o = dst + (j - k) * r + k;
+                if (r == 4) {
+                    const Cd a{v[0].x + v[2].x, v[0].y + v[2].y}, b{v[0].x - v[2].x, v[0].y - v[2].y};
+                    const Cd c{v[1].x + v[3].x, v[1].y + v[3].y}, d{v[1].x - v[3].x, v[1].y - v[3].y};
+                    o[0] = {a.x + c.x, a.y + c.y};
+                    o[2 * ns] = {a.x - c.x, a.y - c.y};
+                    o[ns] = {b.x - sgn * d.y, b.y + sgn * d.x};
+                    o[3 * ns] = {b.x + sgn * d.y, b.y - sgn * d.x};
+                    continue;
+                }
+                for (int q = 0; q < r; q++) {
+                    Cd acc = v[0];
+                    for (int u = 1; u < r; u++) {
+                        Cd t = w[(u * q % r) * rs];
+                        if (sgn > 0) t.y = -t.y;
+                        const Cd p = mul(v[u], t);
+                        acc.x += p.x;
+                        acc.y += p.y;
+                    }
+                    o[q * ns] = acc;
+                }
+            }
+            std::swap(src, dst);
+            ns *= r;
+        }
+        if (src != x.data()) x.swap(tmp);
+    }
+};
+
+// e^{-i pi k^2 / n} and the transform of the wrapped conjugate chirp, over m
+struct Chirp {
+    std::vector<Cd> c, b;
+    Chirp(int n, HostFFT& f) : c(n), b(f.n, Cd{0.0, 0.0}) {
+        for (long long k = 0; k < n; k++) {
+            const double a = M_PI * (double)((k * k) % (2LL * n)) / (double)n;
+            c[k] = {std::cos(a), -std::sin(a)};
+        }
+        for (int k = 0; k < n; k++) b[k] = {c[k].x, -c[k].y};
+        for (int k = 1; k < n; k++) b[f.n - k] = b[k];
+        f.run(b, -1);
+        for (Cd& v : b) v = {v.x / f.n, v.y / f.n};
+    }
+};
+}  // namespace
+
+// What the tables of one plan share.
+struct TableMaker {
+    HostFFT f;
+    Chirp ch;
+    TableMaker(int n, int m) : f(m), ch(n, f) {}
+};
+static TableMaker& maker(const HostPlan& hp) {
+    if (!hp.maker) hp.maker = std::make_shared<TableMaker>(hp.n, hp.m);
+    return *hp.maker;
 }
 
 // Lengths with compiled z passes (ac_kernels.cu, vz_kernels.cu).
@@ -282,19 +342,11 @@ static void plan_twiddles(HostPlan& hp) {
 }
 
 void add_bluestein(HostPlan& hp) {
-    const int n = hp.n, m = hp.m;
-    hp.chirp.resize(n);
-    for (long long k = 0; k < n; k++) {
-        const long long q = (k * k) % (2LL * n);
-        const double a = -M_PI * (double)q / (double)n;
-        hp.chirp[k] = std::complex<double>(std::cos(a), std::sin(a));
-    }
-    std::vector<std::complex<double>> b(m, 0.0);
-    for (int k = 0; k < n; k++) b[k] = std::conj(hp.chirp[k]);
-    for (int k = 1; k < n; k++) b[m - k] = std::conj(hp.chirp[k]);
-    host_fft(b, hp.rad, -1);
-    hp.bhat.resize(m);
-    for (int k = 0; k < m; k++) hp.bhat[k] = b[k] / (double)m;
+    const Chirp& ch = maker(hp).ch;
+    hp.chirp.clear();
+    hp.bhat.clear();
+    for (const Cd& v : ch.c) hp.chirp.emplace_back(v.x, v.y);
+    for (const Cd& v : ch.b) hp.bhat.emplace_back(v.x, v.y);
 }
 
 int build_plan_host(int n, HostPlan& hp) {
@@ -371,20 +423,22 @@ void conv_table(const HostPlan& hp, const std::vector<std::complex<double>>& Hn,
         out = Hn;
         return;
     }
-    // h[d] = sum_k Hn[k] e^{+2 pi i k d / n}, exact phases from (k d) mod n
-    std::vector<std::complex<double>> h(n), e(n);
-    for (int q = 0; q < n; q++) e[q] = std::complex<double>(std::cos(2.0 * M_PI * q / n), std::sin(2.0 * M_PI * q / n));
+    // h[d] = sum_k Hn[k] e^{+2 pi i k d / n} = conj(DFT_n(conj Hn)), by Bluestein's identity on m
+    TableMaker& t = maker(hp);
+    std::vector<Cd> x(m, Cd{0.0, 0.0}), hm(m, Cd{0.0, 0.0});
+    for (int k = 0; k < n; k++) x[k] = mul({Hn[k].real(), -Hn[k].imag()}, t.ch.c[k]);
+    t.f.run(x, -1);
+    for (int k = 0; k < m; k++) x[k] = mul(x[k], t.ch.b[k]);
+    t.f.run(x, +1);
     for (int d = 0; d < n; d++) {
-        std::complex<double> acc = 0.0;
-        for (int k = 0; k < n; k++) acc += Hn[k] * e[(int)(((long long)k * d) % n)];
-        h[d] = acc;
+        const Cd v = mul(x[d], t.ch.c[d]);
+        const Cd h{v.x, -v.y};
+        hm[d] = h;                          // lags 0 .. n-1
+        if (d > 0) hm[m - n + d] = h;       // lags -(n-1) .. -1: slot m - (n - d)
     }
-    std::vector<std::complex<double>> hm(m, 0.0);
-    for (int d = 0; d < n; d++) hm[d] = h[d];               // lags 0 .. n-1
-    for (int d = 1; d < n; d++) hm[m - d] = h[n - d];       // lags -(n-1) .. -1
-    host_fft(hm, hp.rad, -1);
+    t.f.run(hm, -1);
     out.resize(m);
-    for (int k = 0; k < m; k++) out[k] = hm[k] / (double)m;
+    for (int k = 0; k < m; k++) out[k] = std::complex<double>(hm[k].x / m, hm[k].y / m);
 }
 
 int fill_plan_dev(const HostPlan& hp, FFTPlanDev& d) {

@@ -1,6 +1,7 @@
 // host_setup.h -- FP64 coefficient setup and line-FFT plan construction.
 #pragma once
 #include <complex>
+#include <memory>
 #include <vector>
 
 #include "qpstd_internal.h"
@@ -19,12 +20,14 @@ double wavenumber(int i, int n, double d);
 //        2 = z velocity derivative, 3 = z pressure derivative.
 void shift_symbols(int n, double d, int which, std::vector<std::complex<double>>& H, bool raw = false);
 
+struct TableMaker;
 struct HostPlan {
     int n = 0, m = 0, blue = 0;
     int rt = 0;  // entry of rt_list.h (0: a Stockham plan of fft_reg.cuh, one butterfly per thread)
     int wq = 0;  // rt: where the twiddles of the entry's quick form start in w
     std::vector<int> rad;
     std::vector<std::complex<double>> w, chirp, bhat;
+    mutable std::shared_ptr<TableMaker> maker;  // FP64 transforms of the tables, made when first needed
 };
 // Exact DFT plan of a Stockham pass: n itself when it factors into radices <= 16,
 // else Bluestein on a smooth m >= 2n-1.
