@@ -130,15 +130,19 @@ static int put_field(qpstd_shot* s, const float* h, float* f, bool blocked) {
     }
     return QPSTD_OK;
 }
-static int get_window(qpstd_shot* s, const float* f, bool blocked, int nx, int nz, int x0, int z0, float* h) {
+static int field_out(qpstd_shot* s, const float* f, bool blocked, int nx, int nz, int x0, int z0, float* out) {
     const size_t n = (size_t)nx * nz;
+    field_out_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(nx, nz, x0, z0, blocked ? s->rs : s->d.nzz,
+                                                                          blocked ? s->sb : 4, f, out);
+    CK(cudaGetLastError());
+    return QPSTD_OK;
+}
+static int get_window(qpstd_shot* s, const float* f, bool blocked, int nx, int nz, int x0, int z0, float* h) {
     if (blocked || nx != s->d.nxx || nz != s->d.nzz) {
-        field_out_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(nx, nz, x0, z0, blocked ? s->rs : s->d.nzz,
-                                                                              blocked ? s->sb : 4, f, s->io);
-        CK(cudaGetLastError());
+        if (const int rc = field_out(s, f, blocked, nx, nz, x0, z0, s->io)) return rc;
         f = s->io;
     }
-    CK(cudaMemcpyAsync(h, f, sizeof(float) * n, cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaMemcpyAsync(h, f, sizeof(float) * (size_t)nx * nz, cudaMemcpyDeviceToHost, s->stream));
     return QPSTD_OK;
 }
 
@@ -236,7 +240,34 @@ static int build_receivers(qpstd_shot* s, const qpstd_shot_desc* d) {
     return build_rec_list(s, d, 2 * s->Lzv, true, &s->rec_off_z, &s->rec_z);
 }
 
-// Per-point constant-Q coefficients and the spectra scratch (double -> float once).
+// Per-point coefficients from the models (raw: vp, rho, then gam, lam, vwd, tao, N apart), in
+// double, rounded once: c1 = rho vp^2 dt and c2 = (vp dt)^2 / 12 of the acoustic step at their
+// field addresses, and the constant-Q ones (y1, y2, y3c, y4c, e1, e2, e3, N apart).
+__global__ void ac_coef_kernel(int nxx, int nzz, unsigned rs, unsigned sb, size_t N, float dtf, const float* __restrict__ raw,
+                               float* __restrict__ c1, float* __restrict__ c2) {
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (unsigned)nxx * nzz) return;
+    const unsigned ix = i / nzz, iz = i - ix * nzz, o = ix * rs + (iz >> 2) * sb + (iz & 3);
+    const double vp = raw[i], dt = dtf;
+    c1[o] = (float)((double)raw[N + i] * vp * vp * dt);
+    c2[o] = (float)(vp * vp * dt * dt / 12.0);
+}
+__global__ void visco_coef_kernel(int n, size_t N, float dtf, const float* __restrict__ raw, float* __restrict__ f) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double dt = dtf, vp = raw[i], rho = raw[N + i], g = raw[2 * N + i], lam = raw[3 * N + i], w = raw[4 * N + i],
+                 tao = raw[5 * N + i];
+    const double cc = dt * dt * vp * vp * lam / 12.0;  // sum_total, acsglw.cu:1213-1245
+    f[i] = (float)(1.0 - 32.0 * g);
+    f[N + i] = (float)(32.0 * g * w);
+    f[2 * N + i] = (float)((1.0 - 64.0 * g) * cc);
+    f[3 * N + i] = (float)(64.0 * g * w * cc);
+    f[4 * N + i] = (float)(rho * vp * vp * dt * lam);  // addsa_kernel, acsglw.cu:1527
+    f[5 * N + i] = (float)(0.5 * dt * tao);
+    f[6 * N + i] = (float)(dt * tao);
+}
+
+// Per-point constant-Q coefficients and the spectra scratch.
 static int setup_visco(qpstd_shot* s, const qpstd_shot_desc* d) {
     const size_t N = s->N, Nu = (size_t)d->nxx * d->nzz;
     int rc = QPSTD_OK;
@@ -252,21 +283,12 @@ static int setup_visco(qpstd_shot* s, const qpstd_shot_desc* d) {
     for (int k = 0; k < 4; k++) s->spec[k] = reinterpret_cast<float2*>(sp) + k * NS;
     s->src.aux_spec = reinterpret_cast<float2*>(sp) + 4 * NS;
     if (s->rtm) s->rcv.aux_spec = reinterpret_cast<float2*>(sp) + 5 * NS;
-    std::vector<float> h(7 * Nu);
-    const double dt = d->dt;
-    for (size_t i = 0; i < Nu; i++) {
-        const double g = d->gam[i], w = d->vwd[i], vp = d->vp[i], lam = d->lam[i], tao = d->tao[i];
-        const double cc = dt * dt * vp * vp * lam / 12.0;  // sum_total, acsglw.cu:1213-1245
-        h[i] = (float)(1.0 - 32.0 * g);
-        h[Nu + i] = (float)(32.0 * g * w);
-        h[2 * Nu + i] = (float)((1.0 - 64.0 * g) * cc);
-        h[3 * Nu + i] = (float)(64.0 * g * w * cc);
-        h[4 * Nu + i] = (float)((double)d->rho[i] * vp * vp * dt * lam);  // addsa_kernel, acsglw.cu:1527
-        h[5 * Nu + i] = (float)(0.5 * dt * tao);
-        h[6 * Nu + i] = (float)(dt * tao);
-    }
-    for (int k = 0; k < 7; k++)
-        if ((rc = put_field(s, h.data() + (size_t)k * Nu, f + (size_t)k * N, false))) return rc;
+    // vp and rho wait in the wavefield's buffer, the Q fields join them
+    float* raw = s->src.st;
+    const float* q[4] = {d->gam, d->lam, d->vwd, d->tao};
+    for (int k = 0; k < 4; k++) CK(upload(s, raw + (2 + k) * N, q[k], sizeof(float) * Nu));
+    visco_coef_kernel<<<(unsigned)((Nu + 255) / 256), 256, 0, s->stream>>>((int)Nu, N, d->dt, raw, f);
+    CK(cudaGetLastError());
     return QPSTD_OK;
 }
 
@@ -468,19 +490,17 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
 
     // models and per-point coefficients (double -> float once)
     {
-        const size_t Nu = (size_t)nxx * nzz;
-        std::vector<float> c1(Nu), c2(Nu);
-        const double dt = d->dt;
-        for (size_t i = 0; i < Nu; i++) {
-            const double vp = d->vp[i];
-            c1[i] = (float)((double)d->rho[i] * vp * vp * dt);
-            c2[i] = (float)(vp * vp * dt * dt / 12.0);
-        }
-        // c1 in the acoustic x pass, or in z pass C of the low-rank form
+        // c1 in the acoustic x pass, or in z pass C of the low-rank form; the buffer of the
+        // wavefield, zeroed in the end, holds vp and rho for the coefficient kernels
         const bool xc = s->blk && !s->visco;
-        if ((rc = put_field(s, c1.data(), s->c1, xc)) || (rc = put_field(s, c2.data(), s->c2, xc)) ||
-            (rc = put_field(s, d->bbx, s->bbx, s->blk)) || (rc = put_field(s, d->bbz, s->bbz, false)))
-            return bail(rc);
+        const size_t Nu = (size_t)nxx * nzz;
+        float* raw = s->src.st;
+        if ((e = upload(s, raw, d->vp, 4 * Nu)) != cudaSuccess || (e = upload(s, raw + N, d->rho, 4 * Nu)) != cudaSuccess)
+            return bail(cuda_fail(e, "upload"));
+        ac_coef_kernel<<<(unsigned)((Nu + 255) / 256), 256, 0, s->stream>>>(nxx, nzz, xc ? s->rs : nzz, xc ? s->sb : 4, N, d->dt,
+                                                                            raw, s->c1, s->c2);
+        if ((e = cudaGetLastError()) != cudaSuccess) return bail(cuda_fail(e, "coefficients"));
+        if ((rc = put_field(s, d->bbx, s->bbx, s->blk)) || (rc = put_field(s, d->bbz, s->bbz, false))) return bail(rc);
     }
     // 1-D tables
     {
@@ -643,9 +663,22 @@ extern "C" int qpstd_shot_get_state(qpstd_shot* s, float* state) {
     if (!s->blk) {
         CK(cudaMemcpyAsync(state, s->src.st, sizeof(float) * 8 * s->N, cudaMemcpyDeviceToHost, s->stream));
     } else {
+        // the fields in the caller's layout side by side, so that they leave in one copy (eight
+        // copies into memory the host has not touched yet took up to ten times as long); the
+        // buffer is made at the first call and kept
         const size_t n = (size_t)s->d.nxx * s->d.nzz;
-        for (int k = 0; k < 8; k++)
-            if (const int rc = get_window(s, s->src.st + k * s->N, state_blocked(s, k), s->d.nxx, s->d.nzz, 0, 0, state + k * n)) return rc;
+        if (!s->io8 && shot_malloc(s, (void**)&s->io8, sizeof(float) * 8 * n) != cudaSuccess) {
+            s->io8 = nullptr;
+            cudaGetLastError();  // no room: field by field
+        }
+        for (int k = 0; k < 8; k++) {
+            const float* f = s->src.st + k * s->N;
+            int rc = QPSTD_OK;
+            if (s->io8) rc = field_out(s, f, state_blocked(s, k), s->d.nxx, s->d.nzz, 0, 0, s->io8 + k * n);
+            else rc = get_window(s, f, state_blocked(s, k), s->d.nxx, s->d.nzz, 0, 0, state + k * n);
+            if (rc) return rc;
+        }
+        if (s->io8) CK(cudaMemcpyAsync(state, s->io8, sizeof(float) * 8 * n, cudaMemcpyDeviceToHost, s->stream));
     }
     CK(cudaStreamSynchronize(s->stream));
     return QPSTD_OK;
