@@ -25,7 +25,7 @@ extern "C" int qpstd_batch_create(const qpstd_shot_desc* d, int n, qpstd_batch**
     qpstd_batch* b = new qpstd_batch();
     for (int i = 0; i < n; i++) {
         qpstd_shot* s = nullptr;
-        const int rc = qpstd_shot_create(&d[i], &s);
+        const int rc = shot_create_ex(&d[i], &s, true, nullptr, n == 1);
         if (rc) {
             qpstd_batch_destroy(b);
             return rc;

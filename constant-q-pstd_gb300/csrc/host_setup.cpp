@@ -460,6 +460,7 @@ int fill_plan_dev(const HostPlan& hp, FFTPlanDev& d) {
     d.w = d.chirp = d.bhat = nullptr;
     d.rt = hp.rt;
     d.quick = 0;
+    d.pdl = 0;
     if (hp.rt) {  // the entry's own thread count
         d.tx = 32;
         return 0;

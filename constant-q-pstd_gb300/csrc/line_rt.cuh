@@ -233,18 +233,38 @@ template <int R, int S, class T> __device__ __forceinline__ void twiddle(Cx<T> (
     }
 }
 
+// ---- overlap with the kernels before and after on the stream -------------------------------
+// A launch with a programmatic dependency (launch_rt) may start while the kernel before it
+// still runs: everything that kernel writes is read after rt_wait.  rt_release lets the next
+// one start; it then waits beside this kernel's last pass with its tables copied.
+__device__ __forceinline__ void rt_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void rt_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Launches kernel k; pdl: with the programmatic dependency.
+template <class K, class A>
+void launch_rt(K k, unsigned grid, int threads, size_t smem, cudaStream_t s, int pdl, const A& a) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = pdl ? 1 : 0;
+    cudaLaunchKernelEx(&c, k, a);  // the callers check cudaGetLastError
+}
+
 // ---- the engine ------------------------------------------------------------------------
 // PAD: a zero-padded line, inputs and outputs [0, M/2]; else all M.
 // G: line groups (of W lines) per CTA; GF: consecutive threads are consecutive groups (the
 // z passes: neighbouring rows), else consecutive butterflies of a group.  MB: resident
-// CTAs per SM the kernels are compiled for (their register cap).
-template <int W_, bool PAD, bool GF, int G_, int MB, int R1_, int R2_, int R3_> struct LineRT {
+// CTAs per SM the kernels are compiled for (their register cap).  EPI: registers an epilogue
+// loop's loads in flight may take.
+template <int W_, bool PAD, bool GF, int G_, int MB, int R1_, int R2_, int R3_, int EPI> struct LineRT {
     static constexpr int W = W_, G = G_, kMinB = MB, R1 = R1_, R2 = R2_, R3 = R3_;
     static constexpr bool kPad = PAD;
-    // registers an epilogue loop's loads in flight may take: 24 let the z passes run at 96
-    // registers, four CTAs per SM (64-shot batch 10.3 Gpts/s; 48 and three CTAs: 10.0; 16 and five
-    // or six: 9.4 - 9.6, spilling)
-    static constexpr int kEpiRegs = 24;
+    static constexpr int kEpiRegs = EPI;
     using T = typename LineVal<W>::T;
     using C = Cx<T>;
     static constexpr int M = R1 * R2 * R3;

@@ -126,6 +126,7 @@ int put_plan(TableImage& im, const HostPlan& hp, FFTPlanDev& pd) {
     pd.tx = (maxb + 31) / 32 * 32;
     pd.rt = hp.rt;
     pd.quick = 0;
+    pd.pdl = 0;
     pd.w = tw;
     pd.wq = tw + hp.wq;
     pd.chirp = pd.bhat = nullptr;

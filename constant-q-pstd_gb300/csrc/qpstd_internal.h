@@ -45,6 +45,7 @@ struct FFTPlanDev {
     int tx;                // threads per line (>= max B, multiple of 32)
     int rt;                // entry of rt_list.h whose register-to-register passes run this plan (0: none)
     int quick;             // 1: the entry's one-line-per-CTA form
+    int pdl;               // rt: launches overlap with the kernel before (launch_rt, line_rt.cuh)
     FFTPass pass[QP_MAXST];
     const float2* w;       // m twiddles e^{-2 pi i k/m}; rt: the tables of line_rt.cuh
     const float2* wq;      // rt: the same of the quick form

@@ -22,18 +22,18 @@ template <class LR> constexpr size_t smem_many() { return LR::kSmem + (size_t)LR
         default: return false;    \
     }                             \
     return true;
-#define QP_RT_LR using LR = LineRT<W, true, false, G, MB, R1, R2, R3>;
+#define QP_RT_LR using LR = LineRT<W, true, false, G, MB, R1, R2, R3, (QP_RT_GROUP < QP_RT_NWIDE ? kEpiWide : kEpiQuick)>;
 
 template <int W, int G, int MB, int R1, int R2, int R3> void l_xpass(const AcXArgs& a, cudaStream_t s) {
     QP_RT_LR
     const unsigned grid = x_grid<LR>((a.nzz + 1) / 2);
-    if (a.do_p) rt_xpass_kernel<true, LR><<<grid, LR::kThreads, LR::kSmem, s>>>(a);
-    else rt_xpass_kernel<false, LR><<<grid, LR::kThreads, LR::kSmem, s>>>(a);
+    if (a.do_p) launch_rt(rt_xpass_kernel<true, LR>, grid, LR::kThreads, LR::kSmem, s, a.pl.pdl, a);
+    else launch_rt(rt_xpass_kernel<false, LR>, grid, LR::kThreads, LR::kSmem, s, a.pl.pdl, a);
 }
 template <int W, int G, int MB, int R1, int R2, int R3> void l_xconv(const XconvArgs& a, cudaStream_t s) {
     QP_RT_LR
-    if (a.nout > 1) rt_xconv_kernel<true, LR><<<x_grid<LR>(a.nzh), LR::kThreads, smem_many<LR>(), s>>>(a);
-    else rt_xconv_kernel<false, LR><<<x_grid<LR>(a.nzh), LR::kThreads, LR::kSmem, s>>>(a);
+    if (a.nout > 1) launch_rt(rt_xconv_kernel<true, LR>, x_grid<LR>(a.nzh), LR::kThreads, smem_many<LR>(), s, a.pl.pdl, a);
+    else launch_rt(rt_xconv_kernel<false, LR>, x_grid<LR>(a.nzh), LR::kThreads, LR::kSmem, s, a.pl.pdl, a);
 }
 template <class K> bool up(K k, size_t bytes) {
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess;
@@ -64,11 +64,11 @@ bool g_xconv(const XconvArgs& a, cudaStream_t s) {
 #if QP_RT_GROUP < QP_RT_NWIDE
 template <int W, int G, int MB, int R1, int R2, int R3> void l_xexact(const VxsArgs& a, cudaStream_t s) {
     QP_RT_LR
-    rt_xexact_kernel<LR><<<x_grid<LR>(a.nzh), LR::kThreads, LR::kSmem, s>>>(a);
+    launch_rt(rt_xexact_kernel<LR>, x_grid<LR>(a.nzh), LR::kThreads, LR::kSmem, s, a.pl.pdl, a);
 }
 template <int W, int G, int MB, int R1, int R2, int R3> void l_convtab(const VtabArgs& a, cudaStream_t s) {
     QP_RT_LR
-    rt_convtab_kernel<LR><<<x_grid<LR>(a.nzh), LR::kThreads, LR::kSmem, s>>>(a);
+    launch_rt(rt_convtab_kernel<LR>, x_grid<LR>(a.nzh), LR::kThreads, LR::kSmem, s, 0, a);
 }
 bool g_xexact(const VxsArgs& a, cudaStream_t s) {
 #define C_(ID, W, G, MB, R1, R2, R3, COST) \

@@ -105,6 +105,7 @@ __device__ __forceinline__ void rt_xpass(const AcXArgs& a, float4* smem) {
     const unsigned o0 = (unsigned)(iz0 >> 2) * a.sb + (iz0 & 3);  // point (0, iz0)
     const bool on = LR::act1() && nc > 0;
     const float2* tw = LR::tables(smem, a.pl.w);
+    rt_wait();
     C v[NZ];
 #pragma unroll
     for (int r = 0; r < NZ; r++) v[r] = czero<T>();
@@ -205,6 +206,7 @@ __device__ __forceinline__ void rt_xpass(const AcXArgs& a, float4* smem) {
         LR::tables_ready();
     }
     if (a.do_v) {
+        if (!a.do_dx) rt_release();
         LR::roundtrip(v, s, tw, a.HxP);
         struct In {
             C pp, v0, bb;
@@ -228,6 +230,7 @@ __device__ __forceinline__ void rt_xpass(const AcXArgs& a, float4* smem) {
         fill(a.vx);
     }
     if (a.do_dx) {
+        rt_release();
         LR::roundtrip(v, s, tw, a.HxM);
         struct In {
             C pv;
@@ -279,6 +282,7 @@ template <bool MANY, class LR> __global__ void __launch_bounds__(LR::kThreads, L
     using C = typename LR::C;
     typename LR::E* s = LR::base(rt_smem);
     const float2* tw = LR::tables(rt_smem, a.pl.w);
+    rt_wait();
     typename LR::E* X = reinterpret_cast<typename LR::E*>(reinterpret_cast<char*>(rt_smem) + LR::kSmem) + LR::group() * LR::M;
     const int nxx = a.nxx, nzh = a.nzh;
     const int kz0 = (blockIdx.x * LR::G + LR::group()) * LR::W;
@@ -314,6 +318,7 @@ template <bool MANY, class LR> __global__ void __launch_bounds__(LR::kThreads, L
             }
         }
         if (MANY && b > 0) __syncthreads();  // the last output's values have been read
+        if (b + 1 == (MANY ? a.nout : 1)) rt_release();
         LR::inverse(x, s, tw, v);
         float2* out = a.out + b * a.out_step;
         rt_rows<LR, LR::NZ>(nxx + z, a.srs + z, o0, on, [&](unsigned, int) { return 0; },
@@ -353,6 +358,7 @@ template <class LR> __global__ void __launch_bounds__(LR::kThreads, LR::kMinB) r
     extern __shared__ float4 rt_smem[];
     using T = typename LR::T;
     const float2* tw = LR::tables(rt_smem, a.pl.w);
+    rt_wait();
     typename LR::E* s = LR::base(rt_smem);
     const int kz0 = (blockIdx.x * LR::G + LR::group()) * LR::W;
     const unsigned o0 = (unsigned)(kz0 >> 1) * a.ssb + (kz0 & 1);
@@ -371,6 +377,7 @@ template <class LR> __global__ void __launch_bounds__(LR::kThreads, LR::kMinB) r
                            sy.y = spec_symbol(a, 0, kx2 + a.kz2[min(kz0 + 1, a.nzz - 1)]) * a.norm;
                        v[r] = cmuls(v[r], sy);
                    });
+    rt_release();
     rt_blue<1, LR>(v, s, a.pl, tw);
     rt_rows<LR, LR::NZ>(a.nxx, a.srs, o0, on, [&](unsigned, int) { return 0; },
                         [&](int r, int, unsigned i, int) { st_spec(a.out0 + i, v[r]); });

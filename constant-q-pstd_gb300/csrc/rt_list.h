@@ -32,10 +32,10 @@
 #define QP_RT_G6(X) X(14, 2, 1, 2, 16, 16, 16, 930) X(15, 1, 1, 2, 16, 20, 16, 1140)
 #define QP_RT_G7(X) X(16, 1, 1, 1, 24, 16, 16, 1400) X(17, 1, 1, 1, 20, 18, 20, 1470)
 #define QP_RT_G8(X) X(18, 1, 1, 1, 24, 18, 20, 1460) X(19, 1, 1, 1, 24, 16, 24, 1460)
-#define QP_RT_G9(X) X(1, 1, 1, 8, 10, 1, 16, 0) X(2, 1, 1, 8, 16, 1, 16, 0) X(3, 1, 1, 8, 8, 6, 8, 0) X(4, 1, 1, 8, 8, 8, 8, 0) X(5, 1, 1, 6, 8, 12, 8, 0)
-#define QP_RT_G10(X) X(6, 1, 1, 5, 8, 16, 8, 0) X(7, 1, 1, 4, 8, 16, 10, 0) X(8, 1, 1, 4, 8, 16, 12, 0)
-#define QP_RT_G11(X) X(9, 1, 1, 4, 8, 16, 16, 0) X(10, 1, 1, 3, 12, 12, 16, 0) X(11, 1, 1, 3, 16, 10, 16, 0)
-#define QP_RT_G12(X) X(12, 1, 1, 3, 16, 12, 16, 0) X(13, 1, 1, 3, 16, 14, 15, 0) X(14, 1, 1, 3, 16, 16, 16, 0)
+#define QP_RT_G9(X) X(1, 1, 1, 8, 8, 4, 5, 0) X(2, 1, 1, 8, 8, 4, 8, 0) X(3, 1, 1, 8, 8, 6, 8, 0) X(4, 1, 1, 8, 8, 8, 8, 0) X(5, 1, 1, 5, 8, 12, 8, 0)
+#define QP_RT_G10(X) X(6, 1, 1, 4, 8, 16, 8, 0) X(7, 1, 1, 3, 8, 16, 10, 0) X(8, 1, 1, 2, 8, 16, 12, 0)
+#define QP_RT_G11(X) X(9, 1, 1, 2, 8, 16, 16, 0) X(10, 1, 1, 2, 12, 12, 16, 0) X(11, 1, 1, 2, 16, 10, 16, 0)
+#define QP_RT_G12(X) X(12, 1, 1, 2, 16, 12, 16, 0) X(13, 1, 1, 2, 16, 14, 15, 0) X(14, 1, 1, 2, 16, 16, 16, 0)
 #define QP_RTZ_G0(X) X(1, 1, 0, 1, 8, 4, 15, 1, 12, 1000) X(2, 1, 0, 1, 8, 3, 10, 1, 20, 1110) X(3, 1, 0, 1, 8, 4, 16, 1, 16, 700)
 #define QP_RTZ_G1(X) X(4, 1, 0, 1, 4, 4, 8, 5, 8, 1100) X(5, 1, 0, 1, 4, 3, 10, 5, 8, 1200) X(6, 1, 0, 1, 2, 5, 8, 8, 8, 1050)
 #define QP_RTZ_G2(X) X(7, 1, 0, 1, 2, 4, 8, 8, 10, 1150) X(8, 1, 0, 1, 2, 4, 11, 6, 10, 1600)
@@ -47,9 +47,9 @@
 #define QP_RTZ_G8(X) X(20, 1, 1, 0, 1, 4, 16, 10, 16, 1250) X(21, 1, 1, 0, 1, 3, 16, 12, 16, 1250)
 #define QP_RTZ_G9(X) X(22, 1, 1, 0, 1, 2, 16, 16, 16, 1150) X(23, 1, 1, 0, 1, 2, 16, 20, 16, 1140)
 #define QP_RTZ_G10(X) X(24, 1, 1, 0, 1, 1, 24, 16, 16, 1400)
-#define QP_RTZ_G11(X) X(1, 1, 0, 0, 1, 4, 15, 1, 12, 0) X(2, 1, 0, 0, 1, 4, 10, 1, 20, 0) X(3, 1, 0, 0, 1, 4, 16, 1, 16, 0) X(4, 1, 0, 0, 1, 4, 8, 5, 8, 0) X(5, 1, 0, 0, 1, 4, 10, 5, 8, 0)
+#define QP_RTZ_G11(X) X(1, 1, 0, 0, 1, 4, 5, 6, 6, 0) X(2, 1, 0, 0, 1, 4, 5, 5, 8, 0) X(3, 1, 0, 0, 1, 4, 8, 4, 8, 0) X(4, 1, 0, 0, 1, 4, 8, 5, 8, 0) X(5, 1, 0, 0, 1, 4, 10, 5, 8, 0)
 #define QP_RTZ_G12(X) X(6, 1, 0, 0, 1, 4, 8, 8, 8, 0) X(7, 1, 0, 0, 1, 4, 8, 8, 10, 0) X(8, 1, 0, 0, 1, 4, 11, 6, 10, 0) X(9, 1, 0, 0, 1, 4, 10, 8, 10, 0)
-#define QP_RTZ_G13(X) X(10, 1, 1, 0, 1, 4, 10, 1, 16, 0) X(11, 1, 1, 0, 1, 4, 16, 1, 16, 0) X(12, 1, 1, 0, 1, 4, 8, 6, 8, 0) X(13, 1, 1, 0, 1, 4, 8, 8, 8, 0)
+#define QP_RTZ_G13(X) X(10, 1, 1, 0, 1, 4, 8, 4, 5, 0) X(11, 1, 1, 0, 1, 4, 8, 4, 8, 0) X(12, 1, 1, 0, 1, 4, 8, 6, 8, 0) X(13, 1, 1, 0, 1, 4, 8, 8, 8, 0)
 #define QP_RTZ_G14(X) X(14, 1, 1, 0, 1, 4, 8, 12, 8, 0) X(15, 1, 1, 0, 1, 4, 8, 16, 8, 0)
 #define QP_RT_WIDE_ALL(X) \
     QP_RT_G0(X) QP_RT_G1(X) QP_RT_G2(X) QP_RT_G3(X) QP_RT_G4(X) QP_RT_G5(X) QP_RT_G6(X) QP_RT_G7(X) QP_RT_G8(X)
@@ -64,6 +64,11 @@
 #define QP_RT_NGROUPS 13
 #define QP_RTZ_NWIDE 11
 #define QP_RTZ_NGROUPS 15
+
+// Registers that an epilogue loop's loads in flight may take.  Wide: 24 let the z passes run at
+// 96 registers, four CTAs per SM (64-shot batch 10.3 Gpts/s; 48 and three CTAs: 10.0; 16 and five
+// or six: 9.4 - 9.6, spilling).  Quick: registers are plenty and each round of loads is a wait.
+constexpr int kEpiWide = 24, kEpiQuick = 96;
 
 // An entry's complex lines per CTA, length and radices (m = 0: no such entry).
 struct RtEntry {

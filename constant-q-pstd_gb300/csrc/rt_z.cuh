@@ -201,6 +201,7 @@ template <class LR> struct ZDft {
     typename LR::E* s = LR::base(rt_smem);                                  \
     const ZRows<LR> z(a.nxx, a.nzz, a.rs, a.sb, a.rz);                            \
     const float2* tw = LR::tables(rt_smem, a.pl.w);                         \
+    rt_wait();                                                              \
     C v[LR::NZ];
 
 // vz <- vz + dt bbz (d + psi), v <- the new vz
@@ -257,6 +258,7 @@ template <class LR> __global__ void __launch_bounds__(LR::kThreads, LR::kMinB) r
     LR::roundtrip(v, s, tw, a.HzM);
     rt_z_div<false, LR>(a, z, v);
     z.clip(v);
+    rt_release();
     LR::roundtrip(v, s, tw, a.kz2);
     z.template put<false>(v, a.Lz);
 }
@@ -278,6 +280,7 @@ template <class LR> __global__ void __launch_bounds__(LR::kThreads, LR::kMinB) r
     LR::roundtrip(v, s, tw, a.HzM);
     rt_z_div<true, LR>(a, z, v);
     z.clip(v);
+    rt_release();
     D::forward(v, s, a.pl, tw, x);
     D::store(x, s, z, a.G, a.nzh, a.srs, a.ssb);
 }
@@ -311,6 +314,7 @@ template <class LR> __global__ void __launch_bounds__(LR::kThreads, LR::kMinB) r
                z.sto(a.total, o, v[r]);
            });
     z.clip(v);
+    rt_release();
     D::forward(v, s, a.pl, tw, x);
     D::store(x, s, z, a.T, a.nzh, a.srs, a.ssb);
 }
@@ -390,6 +394,7 @@ template <class LR> __global__ void __launch_bounds__(LR::kThreads, LR::kMinB) r
                    z.sto(cmp, o, (sm - t.s) - y);
                });
     }
+    rt_release();
     // half spectrum of the new p for the aux operator, and its staggered z derivative
     if constexpr (LR::kPad) {
         C w[LR::NZ];

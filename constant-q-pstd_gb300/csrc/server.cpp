@@ -171,7 +171,7 @@ int admit(qpstd_server* sv, Req& r, bool alone) {
         if (need > avail) return alone ? QPSTD_ENOMEM : 0;
     }
     qpstd_shot* s = nullptr;
-    int rc = shot_create_ex(&d, &s, false, &sv->arena);
+    int rc = shot_create_ex(&d, &s, false, &sv->arena, false);
     if (rc == QPSTD_ENOMEM && !alone) return 0;  // fragmentation: wait for running shots
     if (rc) return rc;
     r.shot = s;

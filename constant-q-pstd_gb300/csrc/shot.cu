@@ -418,10 +418,10 @@ static int setup_conv(qpstd_shot* s, const qpstd_shot_desc* d) {
 static int autotune(qpstd_shot* s);
 
 extern "C" int qpstd_shot_create(const qpstd_shot_desc* d, qpstd_shot** out) {
-    return shot_create_ex(d, out, true, nullptr);
+    return shot_create_ex(d, out, true, nullptr, true);
 }
 
-int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Arena* arena) {
+int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Arena* arena, bool alone) {
     if (!out) return fail(QPSTD_EINVAL, "null output handle");
     *out = nullptr;
     int rc = validate(d);
@@ -564,6 +564,9 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
             if (build_plan_host(nzz, hz)) return bail(fail(QPSTD_ENOTSUP, "no FFT plan for this length"));
             if ((rc = upload_plan(s, hz, s->pz))) return bail(rc);
         }
+        // A shot that runs alone lets its kernels overlap at their ends; among others the next
+        // kernel's waiting CTAs would hold room that other shots' kernels can use.
+        s->px.pdl = s->pz.pdl = s->pxc.pdl = s->pzc.pdl = alone;
         const int pairs_z = (nxx + 1) / 2, pairs_x = (nzz + 1) / 2;
         // acoustic passes: stage the epilogue inputs when they fit beside the lines
         // (z: 5 fields x 2 rows x nzz floats per line; x: up to 9 fields x 2 columns x nxx)

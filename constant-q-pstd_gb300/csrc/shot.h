@@ -48,8 +48,9 @@ struct qpstd_shot;
 int rtm_begin(qpstd_shot* s);
 int rtm_action(qpstd_shot* s);  // 0: more actions, 1: finished, < 0: error code
 // qpstd_shot_create with options: tune runs the lines-per-CTA autotuner, arena
-// (may be null) supplies the device buffers.
-int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Arena* arena);
+// (may be null) supplies the device buffers; alone: the shot is not one of several that
+// advance together.
+int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Arena* arena, bool alone);
 // Moves the shot to a new stream of CUDA priority prio (after its work so far).
 int shot_set_priority(qpstd_shot* s, int prio);
 // Modeling steps t0 .. t0+n-1 with the gather kept on the device (see shot.cu).
