@@ -13,11 +13,6 @@ size_t ac_xpass_smem(int L, int m, int nxx, int nstaged) {
     return sizeof(float2) * (size_t)L * m + sizeof(float) * (size_t)nstaged * nxx * 2 * L;
 }
 
-// Plans compiled into the acoustic z pass (its convolution plan): 1728 = 12^3
-// (nz 800 + CPML 30: 860 needs the convolution length), 660, 200 (see ZPlans
-// in vz_kernels.cu).
-using AcZPlans = PlanList<CtFFT<12, 12, 12>, CtFFT<11, 10, 6>, CtFFT<5, 5, 8>>;
-
 void launch_ac_zpass(const AcZArgs& a, cudaStream_t s) {
     if (a.pl.rt) {
         rtz_any(a.pl.quick, [&](const RtzGroup& g) { return g.zpass(a, s); });
@@ -26,9 +21,8 @@ void launch_ac_zpass(const AcZArgs& a, cudaStream_t s) {
     const int grid = (a.nxx + 2 * a.L - 1) / (2 * a.L);
     const size_t sm = ac_zpass_smem(a.L, a.pl.m, a.nzz, a.stage);
     const dim3 blk(a.pl.tx, a.L);
-#define L_(FPT) ac_zpass_kernel<FPT><<<grid, blk, sm, s>>>(a)
-    QP_DISPATCH(AcZPlans, a.pl, NoExtraPlan{}, plan_max_radix(a.pl) <= 12, L_);
-#undef L_
+    if (plan_max_radix(a.pl) <= 12) ac_zpass_kernel<RtFFT<12>><<<grid, blk, sm, s>>>(a);
+    else ac_zpass_kernel<RtFFT<16>><<<grid, blk, sm, s>>>(a);
 }
 
 // Every buffer of the pass at 16 bytes (the library's own are; a caller's state may not be).
@@ -68,7 +62,6 @@ int ac_set_smem_limits() {
     };
     z(RtFFT<12>{});
     z(RtFFT<16>{});
-    for_each_plan(AcZPlans{}, z);
     auto x = [&](auto fp) {
         using F = decltype(fp);
         bad |= cudaFuncSetAttribute(ac_xpass_kernel<true, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) !=

@@ -332,7 +332,7 @@ __global__ void __maxnreg__(FP::kMaxRadix <= 12 ? QP_R12_REGS : QP_PASS_REGS) ac
     if (a.do_v) {
         if (!have) {
             if (a.stage) cp_async_wait_prior();  // p (first group) has landed
-            xfill<x_epi_batch<FP>()>(sf, T, ld,
+            xfill<kEpiBatchX>(sf, T, ld,
                                      [&](int g, int ix, int iz) { return a.stage ? S(2, g) : a.p[(size_t)ix * nzz + iz]; });
         }
         __syncthreads();
@@ -341,7 +341,7 @@ __global__ void __maxnreg__(FP::kMaxRadix <= 12 ? QP_R12_REGS : QP_PASS_REGS) ac
         struct VIn {
             float pp, v0, bb, hb, ha;
         };
-        batched_for<x_epi_batch<FP>()>(
+        batched_for<kEpiBatchX>(
             T.t0, T.tot, T.nthr,
             [&](int g) {
                 VIn r{0.f, 0.f, 0.f, 0.f, 0.f};
@@ -384,7 +384,7 @@ __global__ void __maxnreg__(FP::kMaxRadix <= 12 ? QP_R12_REGS : QP_PASS_REGS) ac
                 if (P) cp_async_wait_all();
                 else cp_async_wait_prior();
             }
-            xfill<x_epi_batch<FP>()>(sf, T, ld,
+            xfill<kEpiBatchX>(sf, T, ld,
                                      [&](int g, int ix, int iz) { return a.stage ? S(6, g) : a.vx[(size_t)ix * nzz + iz]; });
         }
         __syncthreads();
@@ -393,7 +393,7 @@ __global__ void __maxnreg__(FP::kMaxRadix <= 12 ? QP_R12_REGS : QP_PASS_REGS) ac
         struct DIn {
             float pv, ib, ia;
         };
-        batched_for<x_epi_batch<FP>()>(
+        batched_for<kEpiBatchX>(
             T.t0, T.tot, T.nthr,
             [&](int g) {
                 DIn r{0.f, 0.f, 0.f};

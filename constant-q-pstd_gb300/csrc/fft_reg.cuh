@@ -273,252 +273,19 @@ __device__ __forceinline__ FFTCtx make_ctx(const FFTPlanDev& pl, FFTPass* s_pass
     return c;
 }
 
-// ---- transform policies ---------------------------------------------------------
-// A pass kernel is compiled for one policy, the way it runs its length-m
-// transforms:
-//   RtFFT<RMAX>  the plan's radices read at run time (any plan the host builds;
-//                one RMAX-entry register array and a radix switch per pass);
-//   CtFFT<Rs...> one plan compiled in, radices Rs in pass order: register
-//                arrays of the exact radix, constant strides, divisors and
-//                twiddle strides, and no switch, so each pass is straight-line
-//                code of its own radix.  The launchers use it when the shot's
-//                plan is one of the compiled ones (the lengths the benchmark
-//                workloads and the convolution-length ladder produce).
-// Both compute the same Stockham passes with the same twiddles, so their
-// results agree to the last bit of the arithmetic order.
+// ---- transform policy -----------------------------------------------------------
+// A pass kernel is compiled for RtFFT<RMAX>: the plan's radices read at run time (any
+// plan the host builds; one RMAX-entry register array and a radix switch per pass).
+// These Stockham passes serve the lines beyond the register-to-register entries
+// (rt_list.h) and the low-rank operator's handle.
 template <int RMAX> struct RtFFT {
     static constexpr int kMaxRadix = RMAX;
-    static constexpr bool kCompiled = false;
-    static constexpr int kLen = 0;  // the length is a run-time value
     template <int S> __device__ __forceinline__ static void run(float2* buf, int ld, const FFTCtx& c, int L) {
         fft_m_impl<S, RMAX>(buf, ld, c.sp, c.nst, c.w, L);
     }
 };
 
-// Hooks of the first and last pass of a compiled transform.  run_io lets the
-// first pass take its inputs from a hook instead of the line (zero padding, a
-// multiplier, another buffer) and hands the outputs of the last pass to a hook
-// (a multiplier, another buffer), which folds the sweep over the line that the
-// same operation costs beside a plain transform -- and that sweep's barrier --
-// into the pass.  The arithmetic is the same as the separate sweep's, so the
-// results agree bit for bit.  kSep: the hook reads (writes) memory other than
-// the line, so that pass needs no barrier between its loads and its stores
-// (no thread of the pass then loads what another one stores).
-struct LineIn {
-    static constexpr bool kSep = false;
-    __device__ __forceinline__ float2 load(const float2* line, int i) const { return line[i]; }
-};
-struct LineOut {
-    static constexpr bool kSep = false, kEarly = false;
-    __device__ __forceinline__ void store(float2* line, int i, float2 v) const { line[i] = v; }
-};
-// entries [n, m) of the line read as zeros (a zero-padded convolution)
-struct ZeroPadIn {
-    static constexpr bool kSep = false;
-    int n;
-    __device__ __forceinline__ float2 load(const float2* line, int i) const {
-        return (i < n) ? line[i] : make_float2(0.f, 0.f);
-    }
-};
-// kEarly: a pure function of (i, v), applied to the outputs in registers before
-// the pass's barrier (its table loads then overlap the barrier wait); the
-// store after the barrier is plain.
-// inputs times a complex multiplier H[i]
-struct MulIn {
-    static constexpr bool kSep = false;
-    const float2* __restrict__ H;
-    __device__ __forceinline__ float2 load(const float2* line, int i) const { return cmul(line[i], __ldg(&H[i])); }
-};
-// outputs times a complex multiplier H[i] (the spectrum of a convolution kernel)
-struct MulOut {
-    static constexpr bool kSep = false, kEarly = true;
-    const float2* __restrict__ H;
-    __device__ __forceinline__ float2 apply(int i, float2 v) const { return cmul(v, __ldg(&H[i])); }
-    __device__ __forceinline__ void store(float2* line, int i, float2 v) const { line[i] = v; }
-};
-// outputs times an even real multiplier stored for 0..m/2 (tk[min(i, m - i)])
-struct EvenScaleOut {
-    static constexpr bool kSep = false, kEarly = true;
-    const float* __restrict__ tk;
-    int m;
-    __device__ __forceinline__ float2 apply(int i, float2 v) const { return cscale(v, __ldg(&tk[min(i, m - i)])); }
-    __device__ __forceinline__ void store(float2* line, int i, float2 v) const { line[i] = v; }
-};
-// outputs to another buffer (dst: this thread's line there)
-struct CopyOut {
-    static constexpr bool kSep = true, kEarly = false;
-    float2* dst;
-    __device__ __forceinline__ void store(float2*, int i, float2 v) const { dst[i] = v; }
-};
-// inputs from another buffer times an even real multiplier
-struct EvenScaleIn {
-    static constexpr bool kSep = true;
-    const float2* src;
-    const float* __restrict__ tk;
-    int m;
-    __device__ __forceinline__ float2 load(const float2*, int i) const {
-        return cscale(src[i], __ldg(&tk[min(i, m - i)]));
-    }
-};
-
-// Compile-time Stockham passes (NS = product of the earlier radices).  TX = 0:
-// one butterfly per thread (the CTA has at least m / R threads per line for
-// every pass); TX > 0: the line has TX threads and a pass of B = m / R
-// butterflies gives thread j the butterflies j, j + TX, ... (NB = ceil(B / TX)
-// of them), all loaded before the pass's barrier, so NB * R <= 16 keeps them
-// in registers.  That is how lines longer than 768 butterflies of the smallest
-// radix (m above about 5000) stay in one CTA.  The first pass loads through
-// `in`, the last one stores through `out`.
-template <int R, int... Rest> constexpr int first_radix() { return R; }
-
-template <int S, int M, int NS, int TX, class In, class Out, int R, int... Rest>
-__device__ __forceinline__ void ct_passes(float2* line, const float2* __restrict__ tw, bool lact, const In& in,
-                                          const Out& out, float2 wpre) {
-    constexpr bool kFirst = NS == 1, kLast = sizeof...(Rest) == 0;
-    static_assert(!(kFirst && kLast && In::kSep && Out::kSep), "a one-pass transform between two other buffers");
-    constexpr bool kSep = (kFirst && In::kSep) || (kLast && Out::kSep);
-    constexpr int B = M / R;
-    constexpr int NB = (TX == 0) ? 1 : (B + TX - 1) / TX;
-    static_assert(NB * R <= 16, "butterflies of one thread must fit its registers");
-    // One butterfly per thread (TX = 0): the next pass's twiddle is loaded at
-    // the start of this pass, so its latency overlaps this pass's work and
-    // barriers (the pass receives its own as wpre).
-    float2 wnext = make_float2(1.f, 0.f);
-    if constexpr (TX == 0 && !kLast) {
-        constexpr int NS2 = NS * R, R2 = first_radix<Rest...>(), B2 = M / R2;
-        const int j = threadIdx.x;
-        if (lact && j < B2) wnext = __ldg(&tw[(j % NS2) * (M / (NS2 * R2))]);
-    }
-    float2 v[NB][R];
-    int k[NB];
-#pragma unroll
-    for (int q = 0; q < NB; q++) {
-        const int j = threadIdx.x + q * TX;
-        k[q] = 0;
-        if (lact && j < B) {
-            if constexpr (NS > 1) k[q] = j % NS;
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                if constexpr (kFirst) v[q][r] = in.load(line, j + r * B);
-                else v[q][r] = line[j + r * B];
-            }
-            if constexpr (NS > 1) {
-                float2 w1 = (TX == 0) ? wpre : __ldg(&tw[k[q] * (M / (NS * R))]);
-                if (S > 0) w1.y = -w1.y;
-                float2 w = w1;
-#pragma unroll
-                for (int r = 1; r < R; r++) {
-                    v[q][r] = cmul(v[q][r], w);
-                    w = cmul(w, w1);
-                }
-            }
-            dft<R, S>(v[q]);
-            if constexpr (kLast && Out::kEarly) {
-                const int base = (j - k[q]) * R + k[q];
-#pragma unroll
-                for (int r = 0; r < R; r++) v[q][r] = out.apply(base + r * NS, v[q][r]);
-            }
-        }
-    }
-    if constexpr (!kSep) __syncthreads();
-#pragma unroll
-    for (int q = 0; q < NB; q++) {
-        const int j = threadIdx.x + q * TX;
-        if (lact && j < B) {
-            const int base = (j - k[q]) * R + k[q];
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                if constexpr (kLast) out.store(line, base + r * NS, v[q][r]);
-                else line[base + r * NS] = v[q][r];
-            }
-        }
-    }
-    __syncthreads();
-    if constexpr (!kLast) ct_passes<S, M, NS * R, TX, In, Out, Rest...>(line, tw, lact, in, out, wnext);
-}
-
-template <int TX, int... Rs> struct CtFFTX {
-    static constexpr int kTX = TX;  // threads per line (0: one butterfly each)
-    static constexpr int kNst = sizeof...(Rs);
-    static constexpr int kRad[kNst] = {Rs...};
-    static constexpr int M = (Rs * ...);
-    static constexpr int kMaxRadix = [] {
-        int r = 0;
-        for (int x : {Rs...}) r = x > r ? x : r;
-        return r;
-    }();
-    static constexpr bool kCompiled = true;
-    static constexpr int kLen = M;
-    template <int S> __device__ __forceinline__ static void run(float2* buf, int ld, const FFTCtx& c, int L) {
-        ct_passes<S, M, 1, TX, LineIn, LineOut, Rs...>(buf + threadIdx.y * ld, c.w, threadIdx.y < L, LineIn{},
-                                                       LineOut{}, make_float2(1.f, 0.f));
-    }
-    // The same transform with first- and last-pass hooks (LineIn .. EvenScaleIn
-    // above).  Caller has synchronised after filling what `in` reads; ends with
-    // a barrier, the result where `out` put it.
-    template <int S, class In, class Out>
-    __device__ __forceinline__ static void run_io(float2* buf, int ld, const FFTCtx& c, int L, const In& in,
-                                                  const Out& out) {
-        ct_passes<S, M, 1, TX, In, Out, Rs...>(buf + threadIdx.y * ld, c.w, threadIdx.y < L, in, out,
-                                               make_float2(1.f, 0.f));
-    }
-    // host: is p exactly this plan (radices and, for TX > 0, threads per line)?
-    static bool matches(const FFTPlanDev& p) {
-        if (p.m != M || p.nst != kNst || (TX > 0 && p.tx != TX)) return false;
-        for (int i = 0; i < kNst; i++)
-            if (p.pass[i].R != kRad[i]) return false;
-        return true;
-    }
-};
-template <int... Rs> using CtFFT = CtFFTX<0, Rs...>;
-
-// A list of compiled plans and its dispatch: first_match calls fn(Policy{})
-// with the first listed plan that p equals and returns true, else false.
-template <class... Ps> struct PlanList {};
-template <class Fn> bool first_match(PlanList<>, const FFTPlanDev&, Fn&&) { return false; }
-template <class P0, class... Ps, class Fn> bool first_match(PlanList<P0, Ps...>, const FFTPlanDev& p, Fn&& fn) {
-    if (P0::matches(p)) {
-        fn(P0{});
-        return true;
-    }
-    return first_match(PlanList<Ps...>{}, p, fn);
-}
-// fn(Policy{}) for every plan of the list (e.g. to set kernel attributes)
-template <class Fn> void for_each_plan(PlanList<>, Fn&&) {}
-template <class P0, class... Ps, class Fn> void for_each_plan(PlanList<P0, Ps...>, Fn&& fn) {
-    fn(P0{});
-    for_each_plan(PlanList<Ps...>{}, fn);
-}
-
-// Launches kernel template K for plan p: a compiled plan when p is one (and
-// every extra plan of the kernel equals it), else the run-time plan.
-#define QP_DISPATCH(LIST, p, same_extra, r12, LAUNCH)                                  \
-    do {                                                                              \
-        const bool ct_ = first_match(LIST{}, p, [&](auto fp_) {                        \
-            using FPc = decltype(fp_);                                                \
-            if (same_extra(FPc{})) {                                                  \
-                LAUNCH(FPc);                                                          \
-            } else if (r12) {                                                         \
-                LAUNCH(RtFFT<12>);                                                    \
-            } else {                                                                  \
-                LAUNCH(RtFFT<16>);                                                    \
-            }                                                                         \
-        });                                                                           \
-        if (!ct_) {                                                                   \
-            if (r12) {                                                                \
-                LAUNCH(RtFFT<12>);                                                    \
-            } else {                                                                  \
-                LAUNCH(RtFFT<16>);                                                    \
-            }                                                                         \
-        }                                                                             \
-    } while (0)
-
-// QP_DISPATCH's same_extra for kernels with one plan
-struct NoExtraPlan {
-    template <class F> bool operator()(F) const { return true; }
-};
-
-// FP: the transform policy (RtFFT / CtFFT above)
+// FP: the transform policy
 template <int S, class FP = RtFFT<16>>
 __device__ __forceinline__ void fft_m(float2* buf, int ld, const FFTCtx& pl, int L) {
     FP::template run<S>(buf, ld, pl, L);
@@ -569,12 +336,6 @@ __device__ __forceinline__ void dft_n(float2* buf, int ld, const FFTCtx& pl, int
 template <class FP = RtFFT<16>>
 __device__ __forceinline__ void roundtrip_conv(float2* buf, int ld, const FFTCtx& pl, int L,
                                                const float2* __restrict__ Hm) {
-    if constexpr (FP::kCompiled) {
-        // zero padding folded into the first forward pass, Hm into the last
-        FP::template run_io<-1>(buf, ld, pl, L, ZeroPadIn{pl.n}, MulOut{Hm});
-        FP::template run<+1>(buf, ld, pl, L);
-        return;
-    }
     const int l = threadIdx.y;
     float2* line = buf + l * ld;
     const bool act = l < L;

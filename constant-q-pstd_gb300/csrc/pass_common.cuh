@@ -42,14 +42,9 @@ __device__ __forceinline__ void batched_for(int k0, int n, int step, LoadF&& loa
         }
     }
 }
-// U of the pass kernels' epilogues: x passes (one field value per point of a
-// row) and z passes (two rows per point, under tighter register caps).  x
-// lines of a compiled length of 2048 or more leave each thread 10 or more
-// points of its tile and take 8 at a time (6 in the radix-12 instances, whose
-// 48-register cap spills at 8); measured on the 5040-point lines of the large
-// RTM grid: 8.8 -> 9.2 Gpts/s, the Q-RTM batch 8.37 -> 8.44.
+// U of the Stockham pass kernels' epilogues: x passes (one field value per point of a
+// row) and z passes (two rows per point, under tighter register caps).
 constexpr int kEpiBatchX = 4, kEpiBatchZ = 2;
-template <class FP> constexpr int x_epi_batch() { return FP::kLen < 2048 ? kEpiBatchX : FP::kMaxRadix <= 12 ? 6 : 8; }
 
 // Compensated accumulation s += v (Kahan), used for the image and the
 // illumination sums over thousands of steps.
@@ -91,21 +86,6 @@ __device__ __forceinline__ void zrepack(const float2* __restrict__ S, float2* li
         line[k] = (k < nzh) ? make_float2(A.x - B.y, A.y + B.x) : make_float2(A.x + B.y, -A.y + B.x);
     }
 }
-
-// zrepack as the load hook of a compiled transform's first pass (fft_reg.cuh,
-// run_io): entry k of the packed line, read straight from the half spectra.
-struct ZRepackIn {
-    static constexpr bool kSep = true;
-    const float2* __restrict__ S;
-    int nzz, nzh, xa;
-    bool has0, has1;
-    __device__ __forceinline__ float2 load(const float2*, int k) const {
-        const int kk = (k < nzh) ? k : nzz - k;
-        const float2 A = has0 ? S[(size_t)xa * nzh + kk] : make_float2(0.f, 0.f);
-        const float2 B = has1 ? S[(size_t)(xa + 1) * nzh + kk] : make_float2(0.f, 0.f);
-        return (k < nzh) ? make_float2(A.x - B.y, A.y + B.x) : make_float2(A.x + B.y, -A.y + B.x);
-    }
-};
 
 // half spectra of rows (xa, xa+1) <- this thread's transformed packed line
 __device__ __forceinline__ void zunpack(const float2* line, float2* __restrict__ S, int nzz, int nzh, bool has0,

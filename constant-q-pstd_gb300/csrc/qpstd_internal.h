@@ -3,17 +3,14 @@
 #include <cuda_runtime.h>
 
 #define QP_MAXST 10
-// Threads per CTA of the pass kernels.  Kernels without a register cap below
-// declare __launch_bounds__(QP_MAXTHREADS, 1), i.e. up to 80 registers.
+// The Stockham pass kernels (lines beyond the entries of rt_list.h) have at most
+// QP_MAXTHREADS threads; without a register cap below they declare
+// __launch_bounds__(QP_MAXTHREADS, 1), i.e. up to 80 registers.
 #define QP_MAXTHREADS 768
-// Register cap of the step's pass kernels: at 56 they compile spill-free and hold
-// 4 (not 3) 256-thread line CTAs, or 9 (not 8) 128-thread ones, per SM (registers
-// are allocated per warp in units of 256), which matters when many shots share
-// the GPU.  The three-output x-spectral pass keeps
-// 80: capped, it measured slower (at 56 without spills, four of its 54 KB CTAs per
-// SM leave too little L1 for its table and twiddle loads).  The exact-DFT
-// x-spectral pass (Bluestein transforms and the Q-RTM filter's exponentials)
-// spills below 72 and takes that cap.
+// Register caps of the Stockham passes: at 56 they compile spill-free and hold 4 (not
+// 3) 256-thread line CTAs, or 9 (not 8) 128-thread ones, per SM (registers are allocated
+// per warp in units of 256).  The low-rank x pass keeps 80; the exact-DFT x-spectral
+// pass (Bluestein transforms and the Q-RTM filter's exponentials) spills below 72.
 #define QP_PASS_REGS 56
 // Passes whose plans use radices up to 12 run a 12-entry register array
 // (fft_reg.cuh) and fit 48 registers spill-free (44 too, with the same 6 register
@@ -178,12 +175,10 @@ struct VzArgsA {
 //   mode 2: one output with the Q-RTM stabilised symbol at time t_filter
 struct VxsArgs {
     int nxx, nzz, nzh, L, mode;
-    FFTPlanDev pl;            // exact length-nxx DFT plan (mode 2)
-    FFTPlanDev plc;           // convolution plan along x (modes 0, 1)
+    FFTPlanDev pl;            // exact length-nxx DFT plan
     const float *kx2, *kz2;   // squared wavenumbers (unnormalised)
     const float2* in;
     float2 *out0, *out1, *out2;
-    const float *tab0, *tab1, *tab2;  // per-kz convolution multipliers, nzh x (plc.m/2+1) (modes 0, 1)
     float norm;               // 1/(nxx*nzz)
     float eta6;               // eta * 1e-6 (mode 2)
     float tao, dt, tt;        // filter tau, dt, nt*dt (mode 2)

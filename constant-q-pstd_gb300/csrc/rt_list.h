@@ -3,14 +3,14 @@
 //
 // x entries are X(ID, W, G, MB, R1, R2, R3, COST): W complex lines per thread, G groups of W
 // lines per CTA, MB CTAs per SM the kernels are compiled for, the radices, and the measured
-// clocks x 1000 per point and roundtrip of one SM (a batch of full SMs).  All of them serve
-// zero-padded lines: an n-point line runs on the entry of length M >= 2n - 1 with the least
-// M x COST.  Radices of powers of two cost least, so the ladder is dense around them: lengths
-// between two entries would cost as much as the next one (900 = 30 x 30: 0.93, 1024 = 32 x 32:
-// 0.73 clocks; 3840: 0.99, 4096: 0.93).  Up to 1024 two passes of radices up to 32 with one
-// line per thread beat three (900: 0.93 against 1.05); above, three passes with two packed
-// lines beat one line (3360: 1.07 against 1.22); beyond 4608 two lines leave no registers
-// for a second CTA (5120: 1.19 against 1.14).
+// clocks x 1000 per point and roundtrip of one SM (loops of roundtrips on full SMs).  All of
+// them serve zero-padded lines: an n-point line runs on the entry of length M >= 2n - 1 with the
+// least M x COST.  Radices of powers of two cost least, so the ladder is dense around them:
+// lengths between two entries would cost as much as the next one (3840: 0.99, 4096: 0.93).
+// Short lines take three passes of radices up to 16: two of radices up to 32 measured 0.74
+// clocks against 0.82 at 1024 points but leave too few threads a line.  Two packed lines per
+// thread beat one up to 4096 points (3360: 1.07 against 1.22); beyond 4608 they leave no
+// registers for a second CTA (5120: 1.19 against 1.14).
 //
 // z entries are X(ID, W, PAD, GF, G, MB, R1, R2, R3, COST): PAD 0 transforms lines of exactly
 // M points, PAD 1 serves n <= (M + 1) / 2 (operators as padded convolutions, exact DFTs by

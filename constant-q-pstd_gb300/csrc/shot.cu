@@ -32,7 +32,6 @@ void launch_vz_xspec(const VxsArgs& a, cudaStream_t s);
 void launch_vz_passB(const VzArgsB& a, cudaStream_t s);
 void launch_vz_passC(const VzArgsC& a, cudaStream_t s);
 void launch_vz_zinv(const VzArgsI& a, cudaStream_t s);
-void launch_vz_xspec_conv(const VxsArgs& a, cudaStream_t s);
 void launch_vz_convtab(const VtabArgs& a, cudaStream_t s);
 void launch_lr_xconv(const LrxArgs& a, cudaStream_t s);
 void launch_lr_zsum(const LrsArgs& a, cudaStream_t s);
@@ -314,12 +313,10 @@ static int setup_ksq(qpstd_shot* s, const qpstd_shot_desc* d) {
 
 // Convolution tables of the stationary constant-Q symbols: a symbol that does
 // not change in time is applied per kz column as a circular convolution along x
-// on the convolution length (one FFT per output after a shared forward FFT),
-// which the register-to-register passes run for every width they plan; Stockham
-// plans do so when nxx is not a smooth length, where the exact transforms would
-// go through Bluestein (two FFTs each).
+// on the convolution length (one FFT per output after a shared forward FFT), in
+// every width the register-to-register passes plan.
 static int setup_xtabs(qpstd_shot* s, const qpstd_shot_desc* d) {
-    if (!s->px.blue && !s->pxc.rt) return QPSTD_OK;
+    if (!s->pxc.rt) return QPSTD_OK;
     int rc = QPSTD_OK;
     const int mc = s->pxc.m, nzh = s->nzh, mh = mc / 2 + 1;  // rows keep the even half
     float* t = dalloc(s, (size_t)4 * nzh * mh, &rc);
@@ -328,7 +325,6 @@ static int setup_xtabs(qpstd_shot* s, const qpstd_shot_desc* d) {
     a.nxx = d->nxx; a.nzz = d->nzz; a.nzh = nzh;
     a.pl = s->px; a.plc = s->pxc; a.kx2 = s->kxsq; a.kz2 = s->kzsq;
     a.norm = (float)(1.0 / ((double)d->nxx * d->nzz));
-    if (!s->pxc.rt) a.L = choose_L(nzh, std::max(s->px.m, mc), std::max(s->px.tx, s->pxc.tx), 1, false);
     for (int k = 0; k < 4; k++) {
         a.sym = k;
         a.out = t + (size_t)k * nzh * mh;
@@ -339,10 +335,6 @@ static int setup_xtabs(qpstd_shot* s, const qpstd_shot_desc* d) {
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "convolution tables");
     s->xconv = true;
-    if (s->pxc.rt) return QPSTD_OK;
-    s->Lxs_exact = s->Lxs;
-    s->Lxs = choose_L(nzh, mc, s->pxc.tx, 1, true);
-    s->Lxs3 = choose_L(nzh, mc, s->pxc.tx, 2, true);
     return QPSTD_OK;
 }
 
@@ -565,7 +557,8 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
             if ((rc = upload_plan(s, hz, s->pz))) return bail(rc);
         }
         // A shot that runs alone lets its kernels overlap at their ends; among others the next
-        // kernel's waiting CTAs would hold room that other shots' kernels can use.
+        // kernel's waiting CTAs would hold room that other shots' kernels can use (16-shot Q-RTM
+        // batch 43.7 ms without, 46.2 with; 439 x 200 acoustic step alone 23.7 us without, 13.6 with).
         s->px.pdl = s->pz.pdl = s->pxc.pdl = s->pzc.pdl = alone;
         const int pairs_z = (nxx + 1) / 2, pairs_x = (nzz + 1) / 2;
         // acoustic passes: stage the epilogue inputs when they fit beside the lines
@@ -879,7 +872,6 @@ static void vz_step(qpstd_shot* s, Wave& w, float src, int t_filter, float eta, 
     }
     VxsArgs xs{};
     xs.nxx = nxx; xs.nzz = nzz; xs.nzh = nzh; xs.pl = s->px; xs.kx2 = s->kxsq; xs.kz2 = s->kzsq; xs.norm = norm;
-    xs.plc = s->pxc;
     XconvArgs xc{};
     xc.nxx = nxx; xc.nzh = nzh; xc.pl = s->pxc;
     xc.srs = xs.srs = s->blk ? 2 : nzh;
@@ -897,12 +889,6 @@ static void vz_step(qpstd_shot* s, Wave& w, float src, int t_filter, float eta, 
             xc.tab_step = (size_t)nzh * (s->pxc.m / 2 + 1);
             ProfScope ps(s, QPSTD_K_XSPEC);
             launch_rt_xconv(xc, st);
-        } else if (s->xconv && a.mode != 2) {
-            a.tab0 = s->xtab[a.mode == 0 ? 0 : 3];
-            a.tab1 = s->xtab[1];
-            a.tab2 = s->xtab[2];
-            ProfScope ps(s, QPSTD_K_XSPEC);
-            launch_vz_xspec_conv(a, st);
         } else {
             ProfScope ps(s, QPSTD_K_XSPEC_EXACT);
             launch_vz_xspec(a, st);
@@ -992,7 +978,6 @@ static void vz_step(qpstd_shot* s, Wave& w, float src, int t_filter, float eta, 
         } else {
             a.mode = 1;
         }
-        if (a.mode == 2 && s->xconv && !s->pxc.rt) a.L = s->Lxs_exact;
         xspec(a);
         w.aux_pending = true;
     }
@@ -1120,14 +1105,11 @@ static std::vector<Knob> shot_knobs(qpstd_shot* s) {
     const size_t vzb = 160 * 1024, acb = QP_SMEM_DYN_MAX;
     if (s->visco) {
         const int mz = std::max(s->pz.m, s->pzc.m), tz = std::max(s->pz.tx, s->pzc.tx);
-        const FFTPlanDev& pxs = s->xconv ? s->pxc : s->px;
         if (!s->pz.rt) knobs.push_back({&s->Lzv, false, tz, (size_t)16 * mz, vzb});  // z passes A-C share L
-        if (!pxs.rt) {
-            knobs.push_back({&s->Lxs3, true, pxs.tx, (size_t)16 * pxs.m, vzb});
-            knobs.push_back({&s->Lxs, true, pxs.tx, (size_t)8 * pxs.m, vzb});
+        if (!s->px.rt) {
+            knobs.push_back({&s->Lxs3, true, s->px.tx, (size_t)16 * s->px.m, vzb});
+            knobs.push_back({&s->Lxs, true, s->px.tx, (size_t)8 * s->px.m, vzb});
         }
-        if (s->xconv && s->d.kind == QPSTD_QRTM && !s->pxc.rt)
-            knobs.push_back({&s->Lxs_exact, true, s->px.tx, (size_t)8 * s->px.m, vzb});
     } else if (!s->pzc.rt) {
         knobs.push_back({&s->Lzp, false, s->pzc.tx, (size_t)8 * s->pzc.m, acb, &s->stage_z, stz});
     }

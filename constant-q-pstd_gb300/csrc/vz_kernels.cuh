@@ -25,17 +25,10 @@ namespace qp {
 
 // this thread's packed line <- the inverse z transform of the half spectra S
 // of rows (xa, xa+1).  The caller has synchronised since the line was last
-// read; ends with a barrier.  With a compiled plan that is not Bluestein the
-// repacking is the first pass's load (no sweep through shared memory first).
+// read; ends with a barrier.
 template <class FP>
 __device__ __forceinline__ void zrepack_inverse(const float2* __restrict__ S, float2* smem, int ld, const FFTCtx& fc,
                                                 int L, int nzz, int nzh, bool has0, bool has1, int xa) {
-    if constexpr (FP::kCompiled) {
-        if (!fc.blue) {
-            FP::template run_io<+1>(smem, ld, fc, L, ZRepackIn{S, nzz, nzh, xa, has0, has1}, LineOut{});
-            return;
-        }
-    }
     zrepack(S, smem + threadIdx.y * ld, nzz, nzh, has0, has1, xa);
     __syncthreads();
     dft_n<+1, FP>(smem, ld, fc, L);
@@ -151,7 +144,7 @@ __global__ void __maxnreg__(FP::kMaxRadix <= 12 ? QP_PASS_REGS : QP_EXACT_REGS) 
     const int nout = (a.mode == 0) ? 3 : 1;
     float2* X = smem + (size_t)L * ld;  // kept forward spectrum (three-output mode)
     float2* line = smem + threadIdx.y * ld;
-    kzfill<x_epi_batch<FP>()>(smem, a.in, ld, L, lg, kz0, nxx, nzh, t0, nthr);
+    kzfill<kEpiBatchX>(smem, a.in, ld, L, lg, kz0, nxx, nzh, t0, nthr);
     __syncthreads();
     dft_n<-1, FP>(smem, ld, fc, L);
     if (nout == 3) {
@@ -188,77 +181,7 @@ __global__ void __maxnreg__(FP::kMaxRadix <= 12 ? QP_PASS_REGS : QP_EXACT_REGS) 
     }
 }
 
-// ---- x-spectral pass, stationary symbols as per-kz convolutions ---------------
-// A stationary symbol s(kx, kz) acts on one kz column as a circular
-// convolution along x, so a zero-padded FFT on the smooth convolution length
-// replaces the exact (Bluestein) DFTs: one forward transform, then per output a
-// multiply by the column's table and one inverse transform.
-// NOUT = 3 (mode 0) or 1 (mode 1): each instance carries only the transforms it runs.
-// FP: transform policy of the convolution plan.
-template <int NOUT, class FP>
-__global__ void __maxnreg__(NOUT == 3 ? QP_WIDE_REGS : FP::kMaxRadix <= 12 ? QP_R12_REGS : QP_PASS_REGS)
-    vz_xspec_conv_kernel(VxsArgs a) {
-    extern __shared__ float2 smem[];
-    __shared__ FFTPass s_pass[QP_MAXST];
-    const FFTCtx fc = make_ctx(a.plc, s_pass);
-    const int L = a.L, m = a.plc.m, ld = m, nxx = a.nxx, nzh = a.nzh;
-    const int lg = 31 - __clz(L);
-    const int kz0 = blockIdx.x * L;
-    const int t0 = threadIdx.y * blockDim.x + threadIdx.x, nthr = blockDim.x * blockDim.y;
-    const int tot = L * nxx;
-    constexpr int nout = NOUT;
-    float2* X = smem + (size_t)L * ld;  // kept forward spectrum (three-output mode)
-    float2* line = smem + threadIdx.y * ld;
-    kzfill<x_epi_batch<FP>()>(smem, a.in, ld, L, lg, kz0, nxx, nzh, t0, nthr);
-    if constexpr (!FP::kCompiled)
-        for (int k = nxx + threadIdx.x; k < m; k += blockDim.x) line[k] = make_float2(0.f, 0.f);
-    __syncthreads();
-    const int kz = min(kz0 + (int)threadIdx.y, nzh - 1);
-    // the multipliers are even in k: rows hold entries 0..m/2
-    const int mh = m / 2 + 1;
-    if constexpr (FP::kCompiled) {
-        // zero padding in the first pass; the last pass either keeps the
-        // spectrum in X (three outputs) or applies the one multiplier
-        if (nout == 3)
-            FP::template run_io<-1>(smem, ld, fc, L, ZeroPadIn{nxx}, CopyOut{X + threadIdx.y * ld});
-        else
-            FP::template run_io<-1>(smem, ld, fc, L, ZeroPadIn{nxx}, EvenScaleOut{a.tab0 + (size_t)kz * mh, m});
-    } else {
-        fft_m<-1, FP>(smem, ld, fc, L);
-        if (nout == 3) {
-            for (int k = threadIdx.x; k < m; k += blockDim.x) X[threadIdx.y * ld + k] = line[k];
-            __syncthreads();
-        }
-    }
-    auto output = [&](const float* __restrict__ tab, float2* out) {
-        const float2* src = (nout == 3) ? X + threadIdx.y * ld : line;
-        const float* tk = tab + (size_t)kz * mh;
-        if constexpr (FP::kCompiled) {
-            // three outputs: the multiplier is applied as the first inverse pass loads X
-            if (nout == 3) FP::template run_io<+1>(smem, ld, fc, L, EvenScaleIn{src, tk, m}, LineOut{});
-            else FP::template run<+1>(smem, ld, fc, L);
-        } else {
-            for (int k = threadIdx.x; k < m; k += blockDim.x) line[k] = cscale(src[k], __ldg(&tk[min(k, m - k)]));
-            __syncthreads();
-            fft_m<+1, FP>(smem, ld, fc, L);
-        }
-        for (int g = t0; g < tot; g += nthr) {
-            const int c = g & (L - 1), ix = g >> lg;
-            if (kz0 + c < nzh) out[(size_t)ix * nzh + kz0 + c] = smem[c * ld + ix];
-        }
-        __syncthreads();
-    };
-    output(a.tab0, a.out0);
-    if (nout == 3) {
-        output(a.tab1, a.out1);
-        output(a.tab2, a.out2);
-    }
-}
-
 // One-time construction of the per-kz convolution multipliers (see VtabArgs).
-// FP: transform policy of both plans (the run-time plan, or one compiled long
-// plan when the exact length's Bluestein plan and the convolution plan are the
-// same length, as the planner makes them for long lines).
 template <class FP>
 __global__ void __launch_bounds__(768, 1) vz_convtab_kernel(VtabArgs a) {
     extern __shared__ float2 smem[];
@@ -471,20 +394,9 @@ __global__ void __maxnreg__(FP::kMaxRadix <= 12 ? QP_R12_REGS : QP_PASS_REGS) vz
     dft_n<-1, FP>(smem, ld, fc, L);
     zunpack(line, a.P, nzz, nzh, has0, has1, xa);
     __syncthreads();
-    if constexpr (FP::kCompiled) {
-        if (!fc.blue) {
-            // the multiplier applied as the first inverse pass loads the line
-            FP::template run_io<+1>(smem, ld, fc, L, MulIn{a.HzP}, LineOut{});
-        } else {
-            for (int k = threadIdx.x; k < nzz; k += blockDim.x) line[k] = cmul(line[k], __ldg(&a.HzP[k]));
-            __syncthreads();
-            dft_n<+1, FP>(smem, ld, fc, L);
-        }
-    } else {
-        for (int k = threadIdx.x; k < nzz; k += blockDim.x) line[k] = cmul(line[k], __ldg(&a.HzP[k]));
-        __syncthreads();
-        dft_n<+1, FP>(smem, ld, fc, L);
-    }
+    for (int k = threadIdx.x; k < nzz; k += blockDim.x) line[k] = cmul(line[k], __ldg(&a.HzP[k]));
+    __syncthreads();
+    dft_n<+1, FP>(smem, ld, fc, L);
     struct VIn {
         float2 pp, v0, bb;
         float hb, ha;
@@ -550,32 +462,21 @@ __global__ void __maxnreg__(QP_WIDE_REGS) lr_xconv_kernel(LrxArgs a) {
     const int tot = L * nxx;
     float2* X = smem + (size_t)L * ld;  // kept forward spectrum
     float2* line = smem + threadIdx.y * ld;
-    kzfill<x_epi_batch<FP>()>(smem, a.in, ld, L, lg, kz0, nxx, nzh, t0, nthr);
-    if constexpr (FP::kCompiled) {
-        // zero padding in the first pass, the spectrum straight into X
-        __syncthreads();
-        FP::template run_io<-1>(smem, ld, fc, L, ZeroPadIn{nxx}, CopyOut{X + threadIdx.y * ld});
-    } else {
-        for (int k = nxx + threadIdx.x; k < m; k += blockDim.x) line[k] = make_float2(0.f, 0.f);
-        __syncthreads();
-        fft_m<-1, FP>(smem, ld, fc, L);
-        for (int k = threadIdx.x; k < m; k += blockDim.x) X[threadIdx.y * ld + k] = line[k];
-    }
+    kzfill<kEpiBatchX>(smem, a.in, ld, L, lg, kz0, nxx, nzh, t0, nthr);
+    for (int k = nxx + threadIdx.x; k < m; k += blockDim.x) line[k] = make_float2(0.f, 0.f);
+    __syncthreads();
+    fft_m<-1, FP>(smem, ld, fc, L);
+    for (int k = threadIdx.x; k < m; k += blockDim.x) X[threadIdx.y * ld + k] = line[k];
     const int kz = min(kz0 + (int)threadIdx.y, nzh - 1);
     const int mh = m / 2 + 1;
 #pragma unroll 1
     for (int b = 0; b < a.row; b++) {
         const float* tk = a.tab + ((size_t)b * nzh + kz) * mh;
         __syncthreads();
-        if constexpr (FP::kCompiled) {
-            // the multiplier applied as the first inverse pass loads X
-            FP::template run_io<+1>(smem, ld, fc, L, EvenScaleIn{X + threadIdx.y * ld, tk, m}, LineOut{});
-        } else {
-            for (int k = threadIdx.x; k < m; k += blockDim.x)
-                line[k] = cscale(X[threadIdx.y * ld + k], __ldg(&tk[min(k, m - k)]));
-            __syncthreads();
-            fft_m<+1, FP>(smem, ld, fc, L);
-        }
+        for (int k = threadIdx.x; k < m; k += blockDim.x)
+            line[k] = cscale(X[threadIdx.y * ld + k], __ldg(&tk[min(k, m - k)]));
+        __syncthreads();
+        fft_m<+1, FP>(smem, ld, fc, L);
         float2* out = a.out + (size_t)b * nxx * nzh;
         for (int g = t0; g < tot; g += nthr) {
             const int c = g & (L - 1), ix = g >> lg;
@@ -584,37 +485,19 @@ __global__ void __maxnreg__(QP_WIDE_REGS) lr_xconv_kernel(LrxArgs a) {
     }
 }
 
-// z pass of the low-rank pressure term: psc (+)= sum_b c_b(x) q_b(x) over the
-// factors b0 .. b0+nb-1 (nb <= lr_terms<FP>()), q_b the inverse z transform of
-// half spectrum b; the first launch (b0 = 0) overwrites psc.  The factors are
-// written out in sequence like z pass B's terms: a loop around the transform
-// spills registers.  The run-time-plan instances take one factor per launch
-// (three copies of their radix switch spilled 3 KB).
-template <class FP> constexpr int lr_terms() { return FP::kCompiled ? 3 : 1; }
+// z pass of the low-rank pressure term: psc (+)= c_b(x) q_b(x) for factor b, q_b the inverse
+// z transform of half spectrum b; b = 0 overwrites psc.  One factor per launch: copies of
+// the run-time plan's radix switch spill.
 template <class FP>
-__global__ void __maxnreg__(FP::kMaxRadix <= 12 ? QP_R12_REGS : QP_PASS_REGS) lr_zsum_kernel(LrsArgs a, int b0, int nb) {
+__global__ void __maxnreg__(FP::kMaxRadix <= 12 ? QP_R12_REGS : QP_PASS_REGS) lr_zsum_kernel(LrsArgs a, int b) {
     ZPASS_SETUP
     const int nzh = a.nzh;
-    float2* acc = smem + (size_t)(L + threadIdx.y) * ld;
-    auto term = [&](int b, bool first) {
-        zrepack_inverse<FP>(a.Q + (size_t)b * nxx * nzh, smem, ld, fc, L, nzz, nzh, has0, has1, xa);
-        const float* cb = a.c + (size_t)b * nxx * nzz;
-        for (int k = threadIdx.x; k < nzz; k += blockDim.x) {
-            const float2 v = line[k];
-            float2 t = first ? make_float2(0.f, 0.f) : acc[k];
-            if (has0) t.x = fmaf(__ldg(&cb[r0 + k]), v.x, t.x);
-            if (has1) t.y = fmaf(__ldg(&cb[r1 + k]), v.y, t.y);
-            acc[k] = t;
-        }
-        __syncthreads();
-    };
-    term(b0, true);
-    if (lr_terms<FP>() > 1 && nb > 1) term(b0 + 1, false);
-    if (lr_terms<FP>() > 2 && nb > 2) term(b0 + 2, false);
+    zrepack_inverse<FP>(a.Q + (size_t)b * nxx * nzh, smem, ld, fc, L, nzz, nzh, has0, has1, xa);
+    const float* cb = a.c + (size_t)b * nxx * nzz;
     for (int k = threadIdx.x; k < nzz; k += blockDim.x) {
-        const float2 t = acc[k];
-        if (has0) a.psc[r0 + k] = b0 ? a.psc[r0 + k] + t.x : t.x;
-        if (has1) a.psc[r1 + k] = b0 ? a.psc[r1 + k] + t.y : t.y;
+        const float2 v = line[k];
+        if (has0) a.psc[r0 + k] = fmaf(__ldg(&cb[r0 + k]), v.x, b ? a.psc[r0 + k] : 0.f);
+        if (has1) a.psc[r1 + k] = fmaf(__ldg(&cb[r1 + k]), v.y, b ? a.psc[r1 + k] : 0.f);
     }
 }
 
