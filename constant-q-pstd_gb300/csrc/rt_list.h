@@ -65,10 +65,12 @@
 #define QP_RTZ_NWIDE 11
 #define QP_RTZ_NGROUPS 15
 
-// Registers that an epilogue loop's loads in flight may take.  Wide: 24 let the z passes run at
-// 96 registers, four CTAs per SM (64-shot batch 10.3 Gpts/s; 48 and three CTAs: 10.0; 16 and five
-// or six: 9.4 - 9.6, spilling).  Quick: registers are plenty and each round of loads is a wait.
-constexpr int kEpiWide = 24, kEpiQuick = 96;
+// Registers that an epilogue loop's loads in flight may take.  Wide z passes: 36 at 96 registers a
+// thread, four CTAs per SM (z passes of a 4100 x 660 shot 119 us; 24: 121; three CTAs of 128
+// registers 132, which a lone 1678 x 660 shot would like better, 62 against 64.5, and the 64-shot
+// batch worse, 5.68 against 5.36 ms).  Wide x passes: 24 (36 spills on the longest lines: x pass of
+// 4100 x 660 91 -> 99 us).  Quick: registers are plenty and each round of loads is a wait.
+constexpr int kEpiWide = 24, kEpiWideZ = 36, kEpiQuick = 96;
 
 // An entry's complex lines per CTA, length and radices (m = 0: no such entry).
 struct RtEntry {

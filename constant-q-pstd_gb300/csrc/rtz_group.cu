@@ -24,7 +24,7 @@ template <class LR> constexpr size_t smem_sum() { return LR::kSmem + LR::kLines;
 #define QP_RTZ_LAUNCH(NAME, ARGS, K, SMEM)                                                                            \
     template <int W, bool PAD, bool GF, int G, int MB, int R1, int R2, int R3>                             \
     void l_##NAME(const ARGS& a, cudaStream_t s) {                                                                    \
-        using LR = LineRT<W, PAD, GF, G, MB, R1, R2, R3, (QP_RTZ_GROUP < QP_RTZ_NWIDE ? kEpiWide : kEpiQuick)>;                                                              \
+        using LR = LineRT<W, PAD, GF, G, MB, R1, R2, R3, (QP_RTZ_GROUP < QP_RTZ_NWIDE ? kEpiWideZ : kEpiQuick)>;                                                              \
         launch_rt(K<LR>, z_grid<LR>(a.nxx), LR::kThreads, SMEM, s, a.pl.pdl, a);                                                       \
     }
 QP_RTZ_LAUNCH(zpass, AcZArgs, rt_zpass_kernel, LR::kSmem)
@@ -37,7 +37,7 @@ template <class K> bool up(K k, size_t bytes) {
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess;
 }
 template <int W, bool PAD, bool GF, int G, int MB, int R1, int R2, int R3> int l_limits() {
-    using LR = LineRT<W, PAD, GF, G, MB, R1, R2, R3, (QP_RTZ_GROUP < QP_RTZ_NWIDE ? kEpiWide : kEpiQuick)>;
+    using LR = LineRT<W, PAD, GF, G, MB, R1, R2, R3, (QP_RTZ_GROUP < QP_RTZ_NWIDE ? kEpiWideZ : kEpiQuick)>;
     static_assert(smem_sum<LR>() <= QP_SMEM_DYN_MAX, "lines of an entry fit a CTA's shared memory");
     return up(rt_zpass_kernel<LR>, LR::kSmem) | up(rt_passA_kernel<LR>, LR::kSmem) | up(rt_passB_kernel<LR>, smem_sum<LR>()) |
            up(rt_passC_kernel<LR>, LR::kSmem) | up(rt_zsum_kernel<LR>, smem_sum<LR>());
