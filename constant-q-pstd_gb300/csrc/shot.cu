@@ -99,12 +99,15 @@ static cudaError_t upload(qpstd_shot* s, void* dst, const void* h, size_t bytes)
 // When both directions run the register-to-register passes (s->blk), the fields that the x
 // passes touch are blocked: point (ix, iz) at ix rs + (iz / 4) sb + iz % 4, rs = 4, sb = 4 nxx
 // (rt_z.cuh).  The z passes' own fields, and every field of other shots, lie row by row like
-// the caller's arrays.  The conversions copy a window of nx x nz points at (x0, z0).
-__global__ void field_in_kernel(int nx, int nz, unsigned rs, unsigned sb, const float* __restrict__ in, float* __restrict__ f) {
+// the caller's arrays.  field_in_kernel takes a whole field into the blocked layout and zeroes its
+// padding (nzp: nz rounded up to 4), which the x passes transform and update beside the points and
+// which holds NaN after an overflow.  field_out_kernel copies a window of nx x nz points at (x0, z0).
+__global__ void field_in_kernel(int nx, int nz, int nzp, unsigned rs, unsigned sb, const float* __restrict__ in,
+                                float* __restrict__ f) {
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (unsigned)nx * nz) return;
-    const unsigned ix = i / nz, iz = i - ix * nz;
-    f[ix * rs + (iz >> 2) * sb + (iz & 3)] = in[i];
+    if (i >= (unsigned)nx * nzp) return;
+    const unsigned ix = i / nzp, iz = i - ix * nzp;
+    f[ix * rs + (iz >> 2) * sb + (iz & 3)] = iz < (unsigned)nz ? in[ix * nz + iz] : 0.f;
 }
 __global__ void field_out_kernel(int nx, int nz, int x0, int z0, unsigned rs, unsigned sb, const float* __restrict__ f,
                                  float* __restrict__ out) {
@@ -124,7 +127,8 @@ static int put_field(qpstd_shot* s, const float* h, float* f, bool blocked) {
     const size_t n = (size_t)s->d.nxx * s->d.nzz;
     CK(upload(s, blocked ? s->io : f, h, sizeof(float) * n));
     if (blocked) {
-        field_in_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(s->d.nxx, s->d.nzz, s->rs, s->sb, s->io, f);
+        field_in_kernel<<<(unsigned)((s->N + 255) / 256), 256, 0, s->stream>>>(s->d.nxx, s->d.nzz, (s->d.nzz + 3) / 4 * 4, s->rs,
+                                                                               s->sb, s->io, f);
         CK(cudaGetLastError());
     }
     return QPSTD_OK;

@@ -74,3 +74,19 @@ def test_filter_that_changes_every_step(nxx, nzz):
     img, ssg = qpstd.rtm_shot(d, obs)
     assert rel_l2(ssg, ref_ssg) < TOL
     assert rel_l2(img, ref_img) < TOL
+
+
+@pytest.mark.parametrize("kind", [qpstd.APS, qpstd.VAPS])
+@pytest.mark.parametrize("nzz", [27, 29, 30])
+def test_state_after_an_overflow(kind, nzz):
+    """A clean state brings a shot back whose fields have overflowed, at depths with padded rows."""
+    d = _shot(kind, 41, nzz)
+    rng = np.random.default_rng(nzz)
+    st0 = (rng.standard_normal((8, 41, nzz)) * SCALE[:, None, None]).astype(np.float32)
+    sh, new = qpstd.Shot(d), qpstd.Shot(d)
+    sh.set_state(np.full((8, 41, nzz), np.nan, dtype=np.float32))
+    sh.advance(0, 2)
+    for s in (sh, new):
+        s.set_state(st0)
+    np.testing.assert_array_equal(sh.advance(0, 3), new.advance(0, 3))
+    np.testing.assert_array_equal(sh.get_state(), new.get_state())
