@@ -149,12 +149,14 @@ int admit(qpstd_server* sv, Req& r, bool alone) {
     const size_t avail = sv->budget > sv->reserved ? sv->budget - sv->reserved : 0;
     size_t need = 0;
     if (is_rtm(d)) {
-        const double N = (double)d.nxx * d.nzz;
-        const size_t per_snap = (size_t)(32.0 * N) + 256;
-        qpstd_shot_desc d0 = d;
+        // a snapshot's bytes as the sizing counts them (with the padding of the shot's field
+        // layout), and the pool's rounding
+        qpstd_shot_desc d0 = d, d1 = d;
         d0.snaps = 0;
+        d1.snaps = 1;
         const long long base = qpstd_shot_bytes(&d0);
         if (base < 0) return QPSTD_EINVAL;
+        const size_t per_snap = (size_t)(qpstd_shot_bytes(&d1) - base) + 256;
         const int want = d.snaps;
         const int floor_snaps = alone ? 1 : std::min(want, 4);
         int fit = (avail > (size_t)base) ? (int)((avail - (size_t)base) / per_snap) : 0;

@@ -93,6 +93,25 @@ def test_server_small_budget_queues_and_lowers_snapshots():
 
 
 @pytest.mark.gpu
+def test_server_budget_counts_padded_snapshots():
+    """A depth whose fields are padded (201 rows in 204): a budget between two snapshot counts is served with the
+    lower one, over a pool whose padding (64 x 38 KB) exceeds the sizing's slack."""
+    d = W.make_shot(qpstd.ARTM, 381, 181, 10, 70, 0.0005, 25.0, seed=511, snaps=64)
+    assert d["nzz"] == 201
+    o = qpstd.model_shot(dict(d, kind=qpstd.APS))
+    base, one = qpstd.shot_bytes(dict(d, snaps=0)), qpstd.shot_bytes(dict(d, snaps=1))
+    per_snap = one - base
+    assert per_snap == 32 * d["nxx"] * 204
+    sv = qpstd.Server(mem_budget=base + 63 * per_snap + per_snap // 4, max_active=2)
+    rid = sv.submit(d, o)
+    sv.wait()
+    st, _, snaps = sv.status(rid)
+    assert st == 2 and snaps == 63
+    assert _same(sv.result(rid), _alone(dict(d, snaps=snaps), o))
+    sv.close()
+
+
+@pytest.mark.gpu
 def test_shot_bytes_covers_the_allocation():
     import torch
     d = W.make_shot(qpstd.QRTM, 560, 300, 20, 400, 0.001, 20.0, seed=7, snaps=12)
