@@ -89,10 +89,22 @@ cudaError_t shot_malloc(qpstd_shot* s, void** p, size_t bytes) {
     return cudaSuccess;
 }
 
-// Host memory to the device on the shot's stream (h may be reused on return: the
-// runtime stages pageable memory).
+// Host memory to the device on the shot's stream.  The copy may still read h after the call:
+// whether the runtime stages pageable memory first is up to it and the machine (a GPU that reads
+// host page tables need not), so h stays valid until the stream has been waited for.
 static cudaError_t upload(qpstd_shot* s, void* dst, const void* h, size_t bytes) {
     return cudaMemcpyAsync(dst, h, bytes, cudaMemcpyHostToDevice, s->stream);
+}
+// A table built for the copy alone: the shot keeps it until uploads_done.
+template <class T> static cudaError_t upload_table(qpstd_shot* s, void* dst, std::vector<T>&& h) {
+    auto t = std::make_shared<std::vector<T>>(std::move(h));
+    s->pending.push_back(t);
+    return upload(s, dst, t->data(), sizeof(T) * t->size());
+}
+static cudaError_t uploads_done(qpstd_shot* s) {
+    const cudaError_t e = cudaStreamSynchronize(s->stream);
+    s->pending.clear();
+    return e;
 }
 
 // ---- the shot's field layout ---------------------------------------------------------
@@ -156,7 +168,7 @@ static int upload_plan(qpstd_shot* s, const HostPlan& hp, FFTPlanDev& d) {
     const size_t cnt = h.size();
     float2* dptr = nullptr;
     CK(shot_malloc(s, (void**)&dptr, sizeof(float2) * cnt));
-    CK(upload(s, dptr, h.data(), sizeof(float2) * cnt));
+    CK(upload_table(s, dptr, std::move(h)));
     d.w = dptr;
     d.wq = dptr + hp.wq;
     d.chirp = hp.chirp.empty() ? nullptr : dptr + hp.w.size();
@@ -227,11 +239,11 @@ static int build_rec_list(qpstd_shot* s, const qpstd_shot_desc* d, int width, bo
     off[ntile] = (int)flat.size();
     int* doff = nullptr;
     CK(shot_malloc(s, (void**)&doff, sizeof(int) * off.size()));
-    CK(upload(s, doff, off.data(), sizeof(int) * off.size()));
+    CK(upload_table(s, doff, std::move(off)));
     RecEntry* drec = nullptr;
     const size_t nrec = std::max<size_t>(flat.size(), 1);
     CK(shot_malloc(s, (void**)&drec, sizeof(RecEntry) * nrec));
-    if (!flat.empty()) CK(upload(s, drec, flat.data(), sizeof(RecEntry) * flat.size()));
+    if (!flat.empty()) CK(upload_table(s, drec, std::move(flat)));
     *off_out = doff;
     *rec_out = drec;
     return QPSTD_OK;
@@ -309,7 +321,7 @@ static int setup_ksq(qpstd_shot* s, const qpstd_shot_desc* d) {
     }
     float* kk = dalloc(s, k2.size(), &rc);
     if (!kk) return rc;
-    CK(upload(s, kk, k2.data(), sizeof(float) * k2.size()));
+    CK(upload_table(s, kk, std::move(k2)));
     s->kxsq = kk;
     s->kzsq = kk + d->nxx;
     return QPSTD_OK;
@@ -360,7 +372,7 @@ static int setup_plain(qpstd_shot* s, const qpstd_shot_desc* d) {
         *dst[w] = cbase + q;
         for (auto& c : H) hc[q++] = make_float2((float)c.real(), (float)c.imag());
     }
-    CK(upload(s, cbase, hc.data(), sizeof(float2) * nc));
+    CK(upload_table(s, cbase, std::move(hc)));
     return QPSTD_OK;
 }
 
@@ -407,7 +419,7 @@ static int setup_conv(qpstd_shot* s, const qpstd_shot_desc* d) {
         H[j] = k * k / d->nzz;
     }
     put(cz, H, &s->cKz2);
-    CK(upload(s, base, hc.data(), sizeof(float2) * nc));
+    CK(upload_table(s, base, std::move(hc)));
     return QPSTD_OK;
 }
 
@@ -522,7 +534,7 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
             const double k = wavenumber(j, nzz, d->dz);
             h[o++] = (float)(k * k / nzz);
         }
-        if ((e = upload(s, base, h.data(), 4 * nt1)) != cudaSuccess) return bail(cuda_fail(e, "upload"));
+        if ((e = upload_table(s, base, std::move(h))) != cudaSuccess) return bail(cuda_fail(e, "upload"));
         std::vector<std::complex<double>> H;
         const size_t nc = 2 * (size_t)nxx + 2 * nzz;
         std::vector<float2> hc(nc);
@@ -538,7 +550,7 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
             *cdst[w] = cbase + q;
             for (auto& c : H) hc[q++] = make_float2((float)c.real(), (float)c.imag());
         }
-        if ((e = upload(s, cbase, hc.data(), sizeof(float2) * nc)) != cudaSuccess) return bail(cuda_fail(e, "upload"));
+        if ((e = upload_table(s, cbase, std::move(hc))) != cudaSuccess) return bail(cuda_fail(e, "upload"));
     }
     // FFT plans and tile shapes of the fused passes (the plain form uses cuFFT)
     if (d->method == QPSTD_FUSED) {
@@ -621,7 +633,7 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
     s->src.aux_pending = false;
     if ((e = cudaMemsetAsync(s->src.st, 0, sizeof(float) * 9 * N, s->stream)) != cudaSuccess) return bail(cuda_fail(e, "memset"));
     // the uploads have left the host buffers and later work may come on any stream
-    if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) return bail(cuda_fail(e, "create"));
+    if ((e = uploads_done(s)) != cudaSuccess) return bail(cuda_fail(e, "create"));
     *out = s;
     return QPSTD_OK;
 }
@@ -651,7 +663,10 @@ extern "C" int qpstd_shot_set_state(qpstd_shot* s, const float* state) {
     } else {
         const size_t n = (size_t)s->d.nxx * s->d.nzz;
         for (int k = 0; k < 8; k++)
-            if (const int rc = put_field(s, state + k * n, s->src.st + k * s->N, state_blocked(s, k))) return rc;
+            if (const int rc = put_field(s, state + k * n, s->src.st + k * s->N, state_blocked(s, k))) {
+                cudaStreamSynchronize(s->stream);  // earlier fields' copies read the caller's memory
+                return rc;
+            }
     }
     CK(cudaStreamSynchronize(s->stream));
     s->src.aux_pending = false;
@@ -1390,7 +1405,9 @@ extern "C" int qpstd_shot_set_lowrank(qpstd_shot* s, int row, int col, const flo
     float* Q = tab ? dalloc(s, (size_t)row * 2 * nxx * nzh, &rc) : nullptr;
     float* Vd = Q ? dalloc(s, (size_t)row * nxh * nvh, &rc) : nullptr;
     if (!Vd) return rc;
-    std::vector<float> hc((size_t)row * Nu);
+    auto kept = std::make_shared<std::vector<float>>((size_t)row * Nu);
+    s->pending.push_back(kept);
+    std::vector<float>& hc = *kept;
     for (size_t x = 0; x < Nu; x++)
         for (int b = 0; b < row; b++) {
             double acc = 0.0;
@@ -1414,7 +1431,7 @@ extern "C" int qpstd_shot_set_lowrank(qpstd_shot* s, int row, int col, const flo
         a.out = tab + (size_t)b * nzh * mh;
         launch_vz_convtab(a, s->stream);
     }
-    cudaError_t e = cudaStreamSynchronize(s->stream);
+    cudaError_t e = uploads_done(s);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "low-rank tables");
     s->lr_c = c;

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <memory>
 #include <vector>
 
 #include "../../include/qpstd.h"
@@ -66,6 +67,7 @@ struct qpstd_shot {
     bool visco = false, rtm = false;
     cudaStream_t stream = nullptr;
     std::vector<void*> allocs;
+    std::vector<std::shared_ptr<void>> pending;  // host tables whose copies may be under way (upload_table)
     qp::Arena* arena = nullptr;  // device buffers come from here when set (server shots)
     qp::Wave src, rcv;
     float *div = nullptr, *Lz = nullptr;
