@@ -133,17 +133,17 @@ static size_t field_at(const qpstd_shot* s, int ix, int iz) { return (size_t)ix 
 // state fields (p, vx, vz, fipx, fipz, fivxx, fivzz, aux) the x passes touch
 static bool state_blocked(const qpstd_shot* s, int k) { return s->blk && (k == 0 || k == 1 || k == 3 || k == 5); }
 
-// One field of the caller's (nxx * nzz floats) to the device field f, and the window of nx x nz
-// points at (x0, z0) of f back; blocked: f lies blocked.
-static int put_field(qpstd_shot* s, const float* h, float* f, bool blocked) {
-    const size_t n = (size_t)s->d.nxx * s->d.nzz;
-    CK(upload(s, blocked ? s->io : f, h, sizeof(float) * n));
-    if (blocked) {
-        field_in_kernel<<<(unsigned)((s->N + 255) / 256), 256, 0, s->stream>>>(s->d.nxx, s->d.nzz, (s->d.nzz + 3) / 4 * 4, s->rs,
-                                                                               s->sb, s->io, f);
-        CK(cudaGetLastError());
-    }
+// The field in s->io to the blocked field f; one field of the caller's (nxx * nzz floats) to the
+// device field f, and the window of nx x nz points at (x0, z0) of f back; blocked: f lies blocked.
+static int field_in(qpstd_shot* s, float* f) {
+    field_in_kernel<<<(unsigned)((s->N + 255) / 256), 256, 0, s->stream>>>(s->d.nxx, s->d.nzz, (s->d.nzz + 3) / 4 * 4, s->rs,
+                                                                           s->sb, s->io, f);
+    CK(cudaGetLastError());
     return QPSTD_OK;
+}
+static int put_field(qpstd_shot* s, const float* h, float* f, bool blocked) {
+    CK(upload(s, blocked ? s->io : f, h, sizeof(float) * s->d.nxx * s->d.nzz));
+    return blocked ? field_in(s, f) : QPSTD_OK;
 }
 static int field_out(qpstd_shot* s, const float* f, bool blocked, int nx, int nz, int x0, int z0, float* out) {
     const size_t n = (size_t)nx * nz;
@@ -673,30 +673,61 @@ extern "C" int qpstd_shot_set_state(qpstd_shot* s, const float* state) {
     return QPSTD_OK;
 }
 
+// The eight state fields in the caller's layout, side by side at the start of s->src.st (from the
+// first to the last, so that none overwrites a later one), and back (from the last to the first).
+// Through s->io; fields that already lie there stay.
+static int state_pack(qpstd_shot* s, bool pack) {
+    const size_t n = (size_t)s->d.nxx * s->d.nzz, N = s->N;
+    for (int i = 0; i < 8; i++) {
+        const int k = pack ? i : 7 - i;
+        const bool blocked = state_blocked(s, k);
+        float *f = s->src.st + k * N, *c = s->src.st + k * n;
+        if (!blocked && n == N) continue;
+        int rc = QPSTD_OK;
+        if (pack) {
+            if ((rc = field_out(s, f, blocked, s->d.nxx, s->d.nzz, 0, 0, s->io))) return rc;
+            CK(cudaMemcpyAsync(c, s->io, sizeof(float) * n, cudaMemcpyDeviceToDevice, s->stream));
+        } else {
+            CK(cudaMemcpyAsync(s->io, c, sizeof(float) * n, cudaMemcpyDeviceToDevice, s->stream));
+            if (!blocked) CK(cudaMemcpyAsync(f, s->io, sizeof(float) * n, cudaMemcpyDeviceToDevice, s->stream));
+            else if ((rc = field_in(s, f))) return rc;
+        }
+    }
+    return QPSTD_OK;
+}
+
+// The state leaves in one copy: eight copies into memory the host had not touched yet took up to
+// ten times as long (53 MB 22.7 against 2.4 ms).  A state of up to kStateKept bytes is gathered in a
+// buffer made at the first call and kept; a larger one in place, which takes no memory but passes
+// over the fields twice (120 steps of 800 x 2088 and their state 13.8 ms with the buffer, 14.2 in
+// place, 14.6 with a buffer allocated and freed at each call).
 extern "C" int qpstd_shot_get_state(qpstd_shot* s, float* state) {
     if (!s || !state) return fail(QPSTD_EINVAL, "null argument");
-    if (!s->blk) {
-        CK(cudaMemcpyAsync(state, s->src.st, sizeof(float) * 8 * s->N, cudaMemcpyDeviceToHost, s->stream));
-    } else {
-        // the fields in the caller's layout side by side, so that they leave in one copy (eight
-        // copies into memory the host has not touched yet took up to ten times as long); the
-        // buffer is made at the first call and kept
-        const size_t n = (size_t)s->d.nxx * s->d.nzz;
-        if (!s->io8 && shot_malloc(s, (void**)&s->io8, sizeof(float) * 8 * n) != cudaSuccess) {
+    constexpr size_t kStateKept = 128 << 20;
+    const size_t n = (size_t)s->d.nxx * s->d.nzz, bytes = sizeof(float) * 8 * n;
+    const float* from = s->src.st;
+    int rc = QPSTD_OK;
+    bool packed = false;
+    if (s->blk) {
+        if (!s->io8 && bytes <= kStateKept && shot_malloc(s, (void**)&s->io8, bytes) != cudaSuccess) {
             s->io8 = nullptr;
-            cudaGetLastError();  // no room: field by field
+            cudaGetLastError();  // no room: in place
         }
-        for (int k = 0; k < 8; k++) {
-            const float* f = s->src.st + k * s->N;
-            int rc = QPSTD_OK;
-            if (s->io8) rc = field_out(s, f, state_blocked(s, k), s->d.nxx, s->d.nzz, 0, 0, s->io8 + k * n);
-            else rc = get_window(s, f, state_blocked(s, k), s->d.nxx, s->d.nzz, 0, 0, state + k * n);
-            if (rc) return rc;
+        if (s->io8) {
+            for (int k = 0; k < 8 && !rc; k++)
+                rc = field_out(s, s->src.st + k * s->N, state_blocked(s, k), s->d.nxx, s->d.nzz, 0, 0, s->io8 + k * n);
+            from = s->io8;
+        } else {
+            packed = true;
+            rc = state_pack(s, true);
         }
-        if (s->io8) CK(cudaMemcpyAsync(state, s->io8, sizeof(float) * 8 * n, cudaMemcpyDeviceToHost, s->stream));
+        if (rc) return rc;
     }
-    CK(cudaStreamSynchronize(s->stream));
-    return QPSTD_OK;
+    const cudaError_t e = cudaMemcpyAsync(state, from, bytes, cudaMemcpyDeviceToHost, s->stream);
+    if (packed) rc = state_pack(s, false);
+    const cudaError_t e2 = cudaStreamSynchronize(s->stream);
+    if (e != cudaSuccess || e2 != cudaSuccess) return cuda_fail(e != cudaSuccess ? e : e2, "state copy");
+    return rc;
 }
 
 // ---------------------------------------------------------------------------

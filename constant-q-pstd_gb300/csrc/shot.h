@@ -87,7 +87,7 @@ struct qpstd_shot {
     bool blk = false, img_full = false;
     unsigned rs = 0, sb = 0;
     size_t NI = 0;                          // points of img, img_c, ssg, ssg_c
-    float *io = nullptr, *io8 = nullptr;    // io8: the whole state, made when first read
+    float *io = nullptr, *io8 = nullptr;    // io8: the whole state, made when first read (up to 128 MiB)
     bool stage_x = false, stage_z = false;  // acoustic passes stage epilogue inputs
     int* rec_off = nullptr;
     qp::RecEntry* rec = nullptr;

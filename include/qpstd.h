@@ -105,7 +105,8 @@ typedef struct qpstd_shot qpstd_shot;
 /* Uploads the models and builds all coefficient tables and FFT plans. */
 int qpstd_shot_create(const qpstd_shot_desc *d, qpstd_shot **out);
 int qpstd_shot_destroy(qpstd_shot *s);
-/* 8*nxx*nzz host floats in the order of qpstd_model_shot's state. */
+/* 8*nxx*nzz host floats in the order of qpstd_model_shot's state.  Reading a
+ * state of up to 128 MiB keeps as much more device memory for later reads. */
 int qpstd_shot_set_state(qpstd_shot *s, const float *state);
 int qpstd_shot_get_state(qpstd_shot *s, float *state);
 /* Advance nsteps steps starting at step index t0 (source wavelet index).

@@ -127,6 +127,25 @@ def test_shot_bytes_covers_the_allocation():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nz", [1000, 1001, 1003])
+def test_reading_a_large_state_keeps_no_device_memory(nz):
+    """The state comes back as it went in, twice, and the shot is as large as before (depths 1040, 1041, 1043: with and
+    without padded rows)."""
+    import torch
+    d = W.make_shot(qpstd.APS, 4100, nz, 20, 10, 0.001, 20.0, seed=8)
+    sh = qpstd.Shot(d)
+    st = np.random.default_rng(3).standard_normal((8, d["nxx"], d["nzz"])).astype(np.float32)
+    sh.set_state(st)
+    torch.cuda.synchronize()
+    f0 = torch.cuda.mem_get_info()[0]
+    for _ in range(2):
+        np.testing.assert_array_equal(sh.get_state(), st)
+    torch.cuda.synchronize()
+    assert f0 - torch.cuda.mem_get_info()[0] < 4 * 2**20  # the state has 138 MB
+    sh.close()
+
+
+@pytest.mark.gpu
 def test_server_serves_windows_beyond_the_fused_lines_in_plain_form():
     d = W.make_shot(qpstd.APS, 6000, 24, 10, 40, 0.0005, 25.0, seed=9)   # padded width 6021
     assert qpstd.shot_bytes(d) < 0 <= qpstd.shot_bytes(dict(d, method=qpstd.PLAIN))
