@@ -440,6 +440,16 @@ void conv_table(const HostPlan& hp, const std::vector<std::complex<double>>& Hn,
     for (int k = 0; k < m; k++) out[k] = std::complex<double>(hm[k].x / m, hm[k].y / m);
 }
 
+void convtab_tables(const HostPlan& hp, std::vector<double2>& out, ConvTabArgs& a) {
+    const TableMaker& t = maker(hp);
+    out.clear();
+    for (const std::vector<Cd>* v : {&t.f.w, &t.ch.c, &t.ch.b})
+        for (const Cd& c : *v) out.push_back(make_double2(c.x, c.y));
+    a.m = hp.m;
+    a.nrad = (int)t.f.rad.size();
+    std::copy(t.f.rad.begin(), t.f.rad.end(), a.rad);
+}
+
 int fill_plan_dev(const HostPlan& hp, FFTPlanDev& d) {
     d.n = hp.n;
     d.m = hp.m;

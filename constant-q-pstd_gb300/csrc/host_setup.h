@@ -52,6 +52,10 @@ int rt_length(int id, RtAxis axis);
 void conv_table(const HostPlan& hp, const std::vector<std::complex<double>>& Hn,
                 std::vector<std::complex<double>>& out);
 
+// FP64 tables of Bluestein's identity on hp.m for convtab.cu: m roots, n chirp values, m of the
+// chirp's transform; a.m and the radices.
+void convtab_tables(const HostPlan& hp, std::vector<double2>& out, ConvTabArgs& a);
+
 // Device view of a plan without its tables: passes, thread count per line.
 // Returns -1 when a pass needs more threads per line than a CTA holds.
 int fill_plan_dev(const HostPlan& hp, FFTPlanDev& d);

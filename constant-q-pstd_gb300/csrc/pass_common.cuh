@@ -153,16 +153,4 @@ __device__ __forceinline__ float spec_symbol(const VxsArgs& a, int j, float k2) 
     const float den = expf(-a.tao * a.tt * ka) + a.eta6 * expf(a.tao * a.dt * ka);
     return ka - num / den;
 }
-// The stationary symbols of the convolution tables in double (see VtabArgs).
-__device__ __forceinline__ double tab_symbol(const VtabArgs& a, int kx, int kz, double k2) {
-    if (a.sym == 4) {
-        const int hx = (kx < a.nxh) ? kx : a.nxx - kx, hz = min(kz, a.nzz - kz);
-        return a.V[(size_t)hx * (a.nzz / 2 + 1) + hz];
-    }
-    if (a.sym == 1) return k2;
-    if (a.sym == 0) return pow(k2, 1.0 / 32.0);
-    if (a.sym == 2) return pow(k2, 33.0 / 32.0);
-    return pow(k2, 0.505);
-}
-
 }  // namespace qp

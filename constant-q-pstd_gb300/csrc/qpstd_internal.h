@@ -187,15 +187,24 @@ struct VxsArgs {
 
 // Builds the per-kz convolution multipliers of a stationary 2-D symbol:
 // for each kz, h = norm * IDFT_x(sym(kx, kz)) zero-padded and wrapped to
-// plc.m, then out[kz*mh + k] = Re FFT_m(h)[k] / m for k = 0..m/2, mh = m/2+1
+// length m, then out[kz*mh + k] = Re FFT_m(h)[k] / m for k = 0..m/2, mh = m/2+1
 // (h is real and even, so the multipliers are real and even in k).
+// In FP64 on Bluestein's length m of an rt x plan (convtab.cu); tables t = 0, 1, .. are
+// (k^2)^(1/32), k^2, (k^2)^(33/32), (k^2)^0.505 or, with V, the low-rank factors.
+struct ConvTabArgs {
+    int nxx, nzz, nzh, m, nrad;
+    int rad[QP_MAXST];          // radices (2, 3, 4, 5, 7)
+    const double2 *w, *chirp, *bhat;  // m roots, nxx chirp values, m of the chirp's transform / m
+    double dkx, dkz;            // wavenumber steps
+    double scale;               // norm / m
+    const float* V;             // (nxx/2+1) x (nzz/2+1) values of each factor
+    float* out;                 // nzh x (m/2+1) of each table
+};
+// The same of one low-rank factor on Stockham plans.
 struct VtabArgs {
-    int nxx, nzz, nzh, L, sym;  // sym: 0 (k^2)^(1/32), 1 k^2, 2 (k^2)^(33/32), 3 (k^2)^0.505,
-                                //      4 the low-rank factor V (half grid, mirrored in kx)
+    int nxx, nzz, nzh, L;
     FFTPlanDev pl, plc;
-    const float *kx2, *kz2;
-    const float* V;             // sym 4: nxh x (nzz/2+1) values of one factor
-    int nxh;
+    const float* V;             // (nxx/2+1) x (nzz/2+1) values, mirrored to the full grid
     float norm;
     float* out;
 };

@@ -10,13 +10,11 @@
 namespace qp {
 
 // Each launches the kernel on the entry plan.rt and returns true, or launches nothing and
-// returns false when the entry is not in the group; the quick groups have no xexact and
-// convtab.  limits raises the dynamic shared-memory limits (non-zero: failed).
+// returns false when the entry is not in the group; the quick groups have no xexact.  limits raises the dynamic shared-memory limits (non-zero: failed).
 struct RtGroup {
     bool (*xpass)(const AcXArgs& a, cudaStream_t s);
     bool (*xconv)(const XconvArgs& a, cudaStream_t s);
     bool (*xexact)(const VxsArgs& a, cudaStream_t s);
-    bool (*convtab)(const VtabArgs& a, cudaStream_t s);
     int (*limits)();
 };
 struct RtzGroup {

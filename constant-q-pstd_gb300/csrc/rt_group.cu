@@ -44,7 +44,7 @@ template <int W, int G, int MB, int R1, int R2, int R3> int l_limits() {
     bool bad = up(rt_xpass_kernel<true, LR>, LR::kSmem) | up(rt_xpass_kernel<false, LR>, LR::kSmem) |
                up(rt_xconv_kernel<false, LR>, LR::kSmem) | up(rt_xconv_kernel<true, LR>, smem_many<LR>());
 #if QP_RT_GROUP < QP_RT_NWIDE
-    bad |= up(rt_xexact_kernel<LR>, LR::kSmem) | up(rt_convtab_kernel<LR>, LR::kSmem);
+    bad |= up(rt_xexact_kernel<LR>, LR::kSmem);
 #endif
     return bad;
 }
@@ -66,25 +66,14 @@ template <int W, int G, int MB, int R1, int R2, int R3> void l_xexact(const VxsA
     QP_RT_LR
     launch_rt(rt_xexact_kernel<LR>, x_grid<LR>(a.nzh), LR::kThreads, LR::kSmem, s, a.pl.pdl, a);
 }
-template <int W, int G, int MB, int R1, int R2, int R3> void l_convtab(const VtabArgs& a, cudaStream_t s) {
-    QP_RT_LR
-    launch_rt(rt_convtab_kernel<LR>, x_grid<LR>(a.nzh), LR::kThreads, LR::kSmem, s, 0, a);
-}
 bool g_xexact(const VxsArgs& a, cudaStream_t s) {
 #define C_(ID, W, G, MB, R1, R2, R3, COST) \
     case ID: l_xexact<W, G, MB, R1, R2, R3>(a, s); break;
     QP_RT_SWITCH(a.pl.rt, C_)
 #undef C_
 }
-bool g_convtab(const VtabArgs& a, cudaStream_t s) {
-#define C_(ID, W, G, MB, R1, R2, R3, COST) \
-    case ID: l_convtab<W, G, MB, R1, R2, R3>(a, s); break;
-    QP_RT_SWITCH(a.plc.rt, C_)
-#undef C_
-}
 #else
 constexpr bool (*g_xexact)(const VxsArgs&, cudaStream_t) = nullptr;
-constexpr bool (*g_convtab)(const VtabArgs&, cudaStream_t) = nullptr;
 #endif
 int g_limits() {
     int bad = 0;
@@ -97,6 +86,6 @@ int g_limits() {
 }  // namespace
 
 extern const RtGroup QP_RT_CAT2(rt_group_, QP_RT_GROUP);
-const RtGroup QP_RT_CAT2(rt_group_, QP_RT_GROUP) = {g_xpass, g_xconv, g_xexact, g_convtab, g_limits};
+const RtGroup QP_RT_CAT2(rt_group_, QP_RT_GROUP) = {g_xpass, g_xconv, g_xexact, g_limits};
 
 }  // namespace qp

@@ -383,50 +383,4 @@ template <class LR> __global__ void __launch_bounds__(LR::kThreads, LR::kMinB) r
                         [&](int r, int, unsigned i, int) { st_spec(a.out0 + i, v[r]); });
 }
 
-// One-time convolution multipliers (VtabArgs): h = norm DFT_n(symbol column), real and
-// even; wrapped to length M its transform is 2 Re F_M(h[0 .. n-1]) - h[0].
-template <class LR> __global__ void __launch_bounds__(LR::kThreads, LR::kMinB) rt_convtab_kernel(VtabArgs a) {
-    extern __shared__ float4 rt_smem[];
-    using T = typename LR::T;
-    __shared__ T h0[LR::G];
-    const float2* tw = LR::tables(rt_smem, a.plc.w);
-    typename LR::E* s = LR::base(rt_smem);
-    const int kz0 = (blockIdx.x * LR::G + LR::group()) * LR::W;
-    typename LR::C v[LR::NZ], x[LR::R3];
-#pragma unroll
-    for (int r = 0; r < LR::NZ; r++) {
-        v[r] = czero<T>();
-        const int ix = LR::index(r);
-        if (LR::act1() && ix < a.nxx && kz0 < a.nzh) {
-            const double kx2 = a.kx2[ix];
-            v[r].x = bcast<T>((float)tab_symbol(a, ix, kz0, kx2 + a.kz2[kz0]));
-            if constexpr (LR::W == 2) {
-                const int k1 = min(kz0 + 1, a.nzh - 1);
-                v[r].x.y = (float)tab_symbol(a, ix, k1, kx2 + a.kz2[k1]);
-            }
-        }
-    }
-    LR::tables_ready();
-    rt_blue<-1, LR>(v, s, a.plc, tw);
-#pragma unroll
-    for (int r = 0; r < LR::NZ; r++) v[r] = {vmul(v[r].x, bcast<T>(a.norm)), bcast<T>(0.f)};
-    if (LR::live() && LR::bfly() == 0) h0[LR::group()] = v[0].x;
-    LR::forward(v, s, tw, x);  // its barriers order h0 too
-    constexpr int mh = LR::M / 2 + 1;
-    if (LR::act3()) {
-        const T z = h0[LR::group()], im = bcast<T>(1.f / LR::M), two = bcast<T>(2.f);
-#pragma unroll
-        for (int r = 0; r < LR::R3; r++) {
-            const int f = LR::freq(r);
-            const T t = vmul(vsub(vmul(two, x[r].x), z), im);
-            if constexpr (LR::W == 1) {
-                if (f < mh && kz0 < a.nzh) a.out[(size_t)kz0 * mh + f] = t;
-            } else {
-                if (f < mh && kz0 < a.nzh) a.out[(size_t)kz0 * mh + f] = t.x;
-                if (f < mh && kz0 + 1 < a.nzh) a.out[(size_t)(kz0 + 1) * mh + f] = t.y;
-            }
-        }
-    }
-}
-
 }  // namespace qp

@@ -33,6 +33,7 @@ void launch_vz_passB(const VzArgsB& a, cudaStream_t s);
 void launch_vz_passC(const VzArgsC& a, cudaStream_t s);
 void launch_vz_zinv(const VzArgsI& a, cudaStream_t s);
 void launch_vz_convtab(const VtabArgs& a, cudaStream_t s);
+cudaError_t launch_convtab(const ConvTabArgs& a, int ntab, cudaStream_t s);
 void launch_lr_xconv(const LrxArgs& a, cudaStream_t s);
 void launch_lr_zsum(const LrsArgs& a, cudaStream_t s);
 void launch_rt_xconv(const XconvArgs& a, cudaStream_t s);
@@ -334,22 +335,13 @@ static int setup_ksq(qpstd_shot* s, const qpstd_shot_desc* d) {
 static int setup_xtabs(qpstd_shot* s, const qpstd_shot_desc* d) {
     if (!s->pxc.rt) return QPSTD_OK;
     int rc = QPSTD_OK;
-    const int mc = s->pxc.m, nzh = s->nzh, mh = mc / 2 + 1;  // rows keep the even half
-    float* t = dalloc(s, (size_t)4 * nzh * mh, &rc);
+    const size_t rows = (size_t)s->nzh * (s->pxc.m / 2 + 1);  // rows keep the even half
+    float* t = dalloc(s, 4 * rows, &rc);
     if (!t) return rc;
-    VtabArgs a{};
-    a.nxx = d->nxx; a.nzz = d->nzz; a.nzh = nzh;
-    a.pl = s->px; a.plc = s->pxc; a.kx2 = s->kxsq; a.kz2 = s->kzsq;
-    a.norm = (float)(1.0 / ((double)d->nxx * d->nzz));
-    for (int k = 0; k < 4; k++) {
-        a.sym = k;
-        a.out = t + (size_t)k * nzh * mh;
-        s->xtab[k] = a.out;
-        launch_vz_convtab(a, s->stream);
-    }
-    cudaError_t e = cudaStreamSynchronize(s->stream);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(e, "convolution tables");
+    for (int k = 0; k < 4; k++) s->xtab[k] = t + k * rows;
+    ConvTabArgs a = s->ctab;
+    a.out = t;
+    CK(launch_convtab(a, 4, s->stream));
     s->xconv = true;
     return QPSTD_OK;
 }
@@ -382,12 +374,25 @@ static int setup_conv(qpstd_shot* s, const qpstd_shot_desc* d) {
     HostPlan cx, cz;
     if (build_conv_plan_host(d->nxx, cx, kRtX) || build_conv_plan_host(d->nzz, cz, s->blk ? kRtZ : kStockham))
         return fail(QPSTD_ENOTSUP, "no convolution plan for this length");
-    // for the convolution tables and the exact transforms
+    // for the exact transforms
     if (s->visco && cx.rt) add_bluestein(cx);
     if (s->visco && cz.rt && cz.m != cz.n) add_bluestein(cz);
     int rc;
     if ((rc = upload_plan(s, cx, s->pxc))) return rc;
     if ((rc = upload_plan(s, cz, s->pzc))) return rc;
+    if (s->visco && cx.rt) {
+        std::vector<double2> t;
+        ConvTabArgs& a = s->ctab;
+        convtab_tables(cx, t, a);
+        double2* p = nullptr;
+        CK(shot_malloc(s, (void**)&p, sizeof(double2) * t.size()));
+        CK(upload_table(s, p, std::move(t)));
+        a.nxx = d->nxx; a.nzz = d->nzz; a.nzh = s->nzh;
+        a.w = p; a.chirp = p + cx.m; a.bhat = a.chirp + d->nxx;
+        a.dkx = wavenumber(1, d->nxx, d->dx);
+        a.dkz = wavenumber(1, d->nzz, d->dz);
+        a.scale = 1.0 / ((double)d->nxx * d->nzz) / cx.m;
+    }
     const size_t nc = 3 * (size_t)cx.m + 3 * (size_t)cz.m;
     std::vector<float2> hc(nc);
     float2* base = nullptr;
@@ -1304,7 +1309,7 @@ extern "C" long long qpstd_shot_bytes(const qpstd_shot_desc* d) {
     f += 16.0 * (d->nxx + d->nzz);                                     // CPML profiles, squared wavenumbers
     if (visco) {
         f += 8.0 * N + 2.0 * NS * (rtm ? 6 : 5) + 4.0 * (d->nxx + d->nzz);
-        if (fused && (ix || ex.blue)) f += 4.0 * nzh * (cx.m / 2 + 1);         // per-kz convolution tables
+        if (fused && ix) f += 4.0 * nzh * (cx.m / 2 + 1) + 4.0 * (2.0 * cx.m + d->nxx);  // per-kz convolution tables, FP64 tables
     }
     f += (double)d->nt * nr;                                           // gather
     if (rtm) f += (double)d->snaps * 8.0 * N + (double)d->nt * nr + 4.0 * (fused && ix ? N : nx * nz);
@@ -1450,17 +1455,22 @@ extern "C" int qpstd_shot_set_lowrank(qpstd_shot* s, int row, int col, const flo
         if ((rc = put_field(s, hc.data() + (size_t)b * Nu, c + (size_t)b * N, false))) return rc;
     CK(cudaMemsetAsync(Q, 0, sizeof(float) * (size_t)row * 2 * nxx * nzh, s->stream));
     CK(upload(s, Vd, V, sizeof(float) * (size_t)row * nxh * nvh));
-    VtabArgs a{};
-    a.nxx = nxx; a.nzz = nzz; a.nzh = nzh;
-    a.pl = s->px; a.plc = s->pxc; a.kx2 = s->kxsq; a.kz2 = s->kzsq;
-    a.norm = (float)(1.0 / ((double)nxx * nzz));
-    if (!s->pxc.rt) a.L = choose_L(nzh, std::max(s->px.m, mc), std::max(s->px.tx, s->pxc.tx), 1, false);
-    a.sym = 4;
-    a.nxh = nxh;
-    for (int b = 0; b < row; b++) {
-        a.V = Vd + (size_t)b * nxh * nvh;
-        a.out = tab + (size_t)b * nzh * mh;
-        launch_vz_convtab(a, s->stream);
+    if (s->pxc.rt) {
+        ConvTabArgs a = s->ctab;
+        a.V = Vd;
+        a.out = tab;
+        CK(launch_convtab(a, row, s->stream));
+    } else {
+        VtabArgs a{};
+        a.nxx = nxx; a.nzz = nzz; a.nzh = nzh;
+        a.pl = s->px; a.plc = s->pxc;
+        a.norm = (float)(1.0 / ((double)nxx * nzz));
+        a.L = choose_L(nzh, std::max(s->px.m, mc), std::max(s->px.tx, s->pxc.tx), 1, false);
+        for (int b = 0; b < row; b++) {
+            a.V = Vd + (size_t)b * nxh * nvh;
+            a.out = tab + (size_t)b * nzh * mh;
+            launch_vz_convtab(a, s->stream);
+        }
     }
     cudaError_t e = uploads_done(s);
     if (e == cudaSuccess) e = cudaGetLastError();

@@ -102,6 +102,7 @@ struct qpstd_shot {
     // nzh x (pxc.m/2+1) for (k^2)^(1/32), k^2, (k^2)^(33/32), (k^2)^0.505
     bool xconv = false;
     const float* xtab[4] = {nullptr, nullptr, nullptr, nullptr};
+    qp::ConvTabArgs ctab{};                  // what builds them, and those of set_lowrank
     // Q-RTM filter: per eta, the last step at which it rounds to k^1.01 (see filter_is_ka)
     std::vector<std::pair<float, int>> ka_steps;
     // low-rank form of the pressure term (qpstd_shot_set_lowrank): row factors,

@@ -3,6 +3,7 @@
 #include "rt.cuh"
 
 namespace qp {
+int convtab_set_smem_limits();
 
 // ---- launchers -------------------------------------------------------------------
 static size_t lsm(int L, int m, int nbuf) { return sizeof(float2) * (size_t)nbuf * L * m; }
@@ -39,10 +40,6 @@ void launch_rt_xconv(const XconvArgs& a, cudaStream_t s) {
     rt_any(a.pl.quick, [&](const RtGroup& g) { return g.xconv(a, s); });
 }
 void launch_vz_convtab(const VtabArgs& a, cudaStream_t s) {
-    if (a.plc.rt) {
-        rt_any(false, [&](const RtGroup& g) { return g.convtab(a, s); });
-        return;
-    }
     const int grid = (a.nzh + a.L - 1) / a.L;
     const dim3 blk(max(a.pl.tx, a.plc.tx), a.L);
     const size_t sm = lsm(a.L, max(a.pl.m, a.plc.m), 1);
@@ -105,7 +102,7 @@ template <class FP> static int vz_set_limits_one() {
 
 int vz_set_smem_limits() {
     const int lim = 200 * 1024;
-    int bad = vz_set_limits_one<RtFFT<12>>() | vz_set_limits_one<RtFFT<16>>();
+    int bad = vz_set_limits_one<RtFFT<12>>() | vz_set_limits_one<RtFFT<16>>() | convtab_set_smem_limits();
     bad |= cudaFuncSetAttribute(vz_xspec_kernel<RtFFT<12>>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess;
     bad |= cudaFuncSetAttribute(vz_xspec_kernel<RtFFT<16>>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess;
     bad |= cudaFuncSetAttribute(vz_convtab_kernel<RtFFT<16>>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim) != cudaSuccess;

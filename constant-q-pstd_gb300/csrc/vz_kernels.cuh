@@ -193,13 +193,9 @@ __global__ void __launch_bounds__(768, 1) vz_convtab_kernel(VtabArgs a) {
     const int kz = blockIdx.x * L + threadIdx.y;
     const bool valid = kz < a.nzh;
     float2* line = smem + threadIdx.y * ld;
-    const double kzsq = a.kz2[valid ? kz : 0];
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const double k2 = (double)a.kx2[k] + kzsq;
-        double s;
-        s = tab_symbol(a, k, valid ? kz : 0, k2);
-        line[k] = make_float2((float)s, 0.f);
-    }
+    const int hz = valid ? min(kz, a.nzz - kz) : 0;
+    for (int k = threadIdx.x; k < n; k += blockDim.x)
+        line[k] = make_float2(a.V[(size_t)min(k, n - k) * (a.nzz / 2 + 1) + hz], 0.f);
     __syncthreads();
     dft_n<+1, FP>(smem, ld, fe, L);  // sum_k s e^{+2 pi i k d/n}
     // wrap to length m: lags 0..n-1 stay, lags -(n-1)..-1 go to m-n+1..m-1 (m >= 2n-1)
