@@ -25,6 +25,7 @@ struct HostPlan {
     int n = 0, m = 0, blue = 0;
     int rt = 0;  // entry of rt_list.h (0: a Stockham plan of fft_reg.cuh, one butterfly per thread)
     int wq = 0;  // rt: where the twiddles of the entry's quick form start in w
+    double gain[2] = {0.0, 0.0};  // rt: what a roundtrip of the wide, the quick form scales a line by, less 1
     std::vector<int> rad;
     std::vector<std::complex<double>> w, chirp, bhat;
     mutable std::shared_ptr<TableMaker> maker;  // FP64 transforms of the tables, made when first needed
@@ -40,17 +41,19 @@ enum RtAxis { kStockham, kRtX, kRtZ };
 int build_conv_plan_host(int n, HostPlan& hp, RtAxis axis = kStockham);
 // Is there a Stockham plan for an n-point line?
 bool stockham_line(int n);
-// Adds the tables of the exact length-n DFT by Bluestein's identity on hp.m.
-void add_bluestein(HostPlan& hp);
+// Adds the tables of the exact length-n DFT by Bluestein's identity on hp.m; rt: for its wide or
+// quick form.
+void add_bluestein(HostPlan& hp, int quick = 0);
 // The entry of rt_list.h an n-point line runs on (0: none is long enough), whether
 // it runs the entry's quick form for this number of lines, and its lines per CTA.
 int rt_choose(int n, RtAxis axis);
 int rt_quick(int id, RtAxis axis, int lines);
 int rt_lines(int id, RtAxis axis, int quick);
 int rt_length(int id, RtAxis axis);
-// Length-m multiplier of the convolution form of the symbol Hn (1/n folded in).
+// Length-m multiplier of the convolution form of the symbol Hn (1/n folded in); rt: for the
+// entry's wide or quick form.
 void conv_table(const HostPlan& hp, const std::vector<std::complex<double>>& Hn,
-                std::vector<std::complex<double>>& out);
+                std::vector<std::complex<double>>& out, int quick = 0);
 
 // FP64 tables of Bluestein's identity on hp.m for convtab.cu: m roots, n chirp values, m of the
 // chirp's transform; a.m and the radices.

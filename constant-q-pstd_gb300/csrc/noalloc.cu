@@ -210,7 +210,7 @@ extern "C" int qpstd_ac_advance_noalloc(const qpstd_shot_desc* d, const float* v
     const float2* tab[6];  // x velocity, x pressure, z velocity, z pressure derivatives; kx^2; kz^2
     for (int w = 0; w < 4; w++) {
         shift_symbols(w < 2 ? nxx : nzz, w < 2 ? d->dx : d->dz, w, H);
-        conv_table(w < 2 ? cx : cz, H, T);
+        conv_table(w < 2 ? cx : cz, H, T, w < 2 ? px.quick : pz.quick);
         tab[w] = put_complex(im, T);
     }
     for (int a = 0; a < 2; a++) {
@@ -221,7 +221,7 @@ extern "C" int qpstd_ac_advance_noalloc(const qpstd_shot_desc* d, const float* v
             const double k = wavenumber(i, n, sp);
             H[i] = k * k / n;
         }
-        conv_table(a ? cz : cx, H, T);
+        conv_table(a ? cz : cx, H, T, a ? pz.quick : px.quick);
         tab[4 + a] = put_complex(im, T);
     }
     std::vector<double> pmlv[8];  // i_ax, i_bx, i_az, i_bz, h_ax, h_bx, h_az, h_bz

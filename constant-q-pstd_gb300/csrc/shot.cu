@@ -374,9 +374,20 @@ static int setup_conv(qpstd_shot* s, const qpstd_shot_desc* d) {
     HostPlan cx, cz;
     if (build_conv_plan_host(d->nxx, cx, kRtX) || build_conv_plan_host(d->nzz, cz, s->blk ? kRtZ : kStockham))
         return fail(QPSTD_ENOTSUP, "no convolution plan for this length");
+    // the forms of the passes: their tables take back the gain of the form's roundtrip
+    const int pairs_x = (d->nzz + 1) / 2, pairs_z = (d->nxx + 1) / 2;
+    if (cx.rt) {
+        s->qx = rt_quick(cx.rt, kRtX, pairs_x);
+        s->qs = rt_quick(cx.rt, kRtX, s->nzh);
+    }
+    if (cz.rt) s->qz = rt_quick(cz.rt, kRtZ, pairs_z);
+    // z transforms on an entry's own length, forward in one pass and inverse in another: what
+    // happens between them takes back their gain
+    const double zgain = cz.rt && cz.m == cz.n ? cz.gain[s->qz] : 0.0;
+    s->spec_norm = (1.0 - zgain) / ((double)d->nxx * d->nzz);
     // for the exact transforms
     if (s->visco && cx.rt) add_bluestein(cx);
-    if (s->visco && cz.rt && cz.m != cz.n) add_bluestein(cz);
+    if (s->visco && cz.rt && cz.m != cz.n) add_bluestein(cz, s->qz);
     int rc;
     if ((rc = upload_plan(s, cx, s->pxc))) return rc;
     if ((rc = upload_plan(s, cz, s->pzc))) return rc;
@@ -391,7 +402,7 @@ static int setup_conv(qpstd_shot* s, const qpstd_shot_desc* d) {
         a.w = p; a.chirp = p + cx.m; a.bhat = a.chirp + d->nxx;
         a.dkx = wavenumber(1, d->nxx, d->dx);
         a.dkz = wavenumber(1, d->nzz, d->dz);
-        a.scale = 1.0 / ((double)d->nxx * d->nzz) / cx.m;
+        a.scale = s->spec_norm * (1.0 - cx.gain[s->qs]) / cx.m;
     }
     const size_t nc = 3 * (size_t)cx.m + 3 * (size_t)cz.m;
     std::vector<float2> hc(nc);
@@ -400,7 +411,7 @@ static int setup_conv(qpstd_shot* s, const qpstd_shot_desc* d) {
     size_t q = 0;
     std::vector<std::complex<double>> H, T;
     auto put = [&](const HostPlan& hp, const std::vector<std::complex<double>>& sym, const float2** dst) {
-        conv_table(hp, sym, T);
+        conv_table(hp, sym, T, &hp == &cx ? s->qx : s->qz);
         *dst = base + q;
         for (auto& c : T) hc[q++] = make_float2((float)c.real(), (float)c.imag());
     };
@@ -587,12 +598,7 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
         const size_t stz = (size_t)40 * nzz, stx = xstage_bytes(s->visco, nxx);
         s->stage_z = !s->pzc.rt && ((size_t)8 * s->pzc.m + stz) <= (size_t)QP_SMEM_DYN_MAX;
         s->stage_x = !s->pxc.rt && ((size_t)8 * s->pxc.m + stx) <= (size_t)QP_SMEM_DYN_MAX;
-        if (s->pxc.rt) {
-            s->qx = rt_quick(s->pxc.rt, kRtX, pairs_x);
-            s->qs = rt_quick(s->pxc.rt, kRtX, s->nzh);
-        }
         if (s->pzc.rt) {
-            s->qz = rt_quick(s->pzc.rt, kRtZ, pairs_z);
             set_quick(s->pz, s->qz);
             set_quick(s->pzc, s->qz);
         }
@@ -912,7 +918,7 @@ static void vz_step(qpstd_shot* s, Wave& w, float src, int t_filter, float eta, 
     const size_t N = s->N;
     cudaStream_t st = s->stream;
     const int nxx = s->d.nxx, nzz = s->d.nzz, nzh = s->nzh;
-    const float norm = (float)(1.0 / ((double)nxx * nzz));
+    const float norm = (float)s->spec_norm;
     {
         VzArgsA a{};
         a.nxx = nxx; a.nzz = nzz; a.nzh = nzh; a.L = s->Lzv; a.pl = s->pz; a.plc = s->pzc;
@@ -1464,7 +1470,7 @@ extern "C" int qpstd_shot_set_lowrank(qpstd_shot* s, int row, int col, const flo
         VtabArgs a{};
         a.nxx = nxx; a.nzz = nzz; a.nzh = nzh;
         a.pl = s->px; a.plc = s->pxc;
-        a.norm = (float)(1.0 / ((double)nxx * nzz));
+        a.norm = (float)s->spec_norm;
         a.L = choose_L(nzh, std::max(s->px.m, mc), std::max(s->px.tx, s->pxc.tx), 1, false);
         for (int b = 0; b < row; b++) {
             a.V = Vd + (size_t)b * nxh * nvh;

@@ -81,6 +81,7 @@ struct qpstd_shot {
     const float2 *cHxM = nullptr, *cHxP = nullptr, *cKx2 = nullptr;  // convolution multipliers
     const float2 *cHzM = nullptr, *cHzP = nullptr, *cKz2 = nullptr;
     int Lx = 1, Lzp = 1, ntile_x = 0;
+    double spec_norm = 0.0;                 // 1/(nxx nzz), with the gain of exact z transforms taken back
     int qx = 0, qs = 0, qz = 0;             // quick form of the x pass / x-spectral / z passes (rt_list.h)
     // layout of the device fields (rt_z.cuh): blocked or row by row, and their strides; N counts
     // the padding; io: nxx * nzz floats for the conversions from and to the caller's layout

@@ -114,3 +114,19 @@ def test_spectral_operator_error(nxx, nzz):
     ref = np.fft.ifft2(np.fft.fft2(st[0]) * sym).real
     fp32 = sf.ifft2(sf.fft2(st[0].astype(np.complex64)) * sym.astype(np.float32)).real
     assert rel_l2(st[7], ref) < 1.5 * rel_l2(fp32, ref)
+
+
+@pytest.mark.parametrize("nxx,nzz", [(300, 300), (337, 240), (512, 512), (800, 180)])
+def test_illumination_has_no_bias(nxx, nzz):
+    """A homogeneous medium whose coefficients are powers of two (their rounding stays out of it): the illumination is
+    proportional to the fourth power of the wave speed's inverse, so derivatives short by 5e-8 would show as 2e-7.
+    Left by the mean gain that the multipliers take back: 1e-8 a derivative, 4e-8, and as much for rounding."""
+    d = _shot(qpstd.ARTM, nxx, nzz, nt=60, snaps=5, pml=20)
+    one = np.ones(nxx * nzz, dtype=np.float32)
+    d = dict(d, vp=2048 * one, rho=256 * one, bbx=one / 256, bbz=one / 256, dt=2.0 ** -10)
+    obs = np.zeros((d["nt"], len(d["gxg"])))
+    _, ref, _ = O.OracleShot(d).rtm(obs)
+    _, ssg = qpstd.rtm_shot(d, obs)
+    ref, ssg = np.asarray(ref, dtype=np.float64).ravel(), ssg.astype(np.float64).ravel()
+    bias = (ssg * ref).sum() / (ref * ref).sum() - 1
+    assert abs(bias) < 8e-8, bias
