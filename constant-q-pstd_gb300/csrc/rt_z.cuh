@@ -2,43 +2,34 @@
 // same steps as ac_zpass_kernel (ac_kernels.cuh) and the z passes of the constant-Q step
 // (vz_kernels.cuh).
 //
-// A line packs x rows as real and imaginary parts: W = 1 rows (0, 1) of its group's pair,
-// W = 2 rows (0, 2) and (1, 3) of four.  Point (ix, iz) of a field that both directions touch
-// (p, Dx; acoustic also div, Lz) sits at (iz / 4) sb + iz % 4 + ix rs: blocked (rs = 4,
-// sb = 4 nxx), where an x pass's rows are contiguous and a CTA of 4 z rows touches 64-byte
-// pieces, or row by row (rs = nzz, sb = 4).  The fields of one direction lie its way: the x
-// pass's blocked, the z passes' row by row (rz = nzz).  Measured with every field row by row:
-// the x passes of a 1678 x 660 shot 45 against 32 us, 2461 x 860 161 against 94; with every
-// field blocked the z passes lose more than that.  Half spectra: (ix, kz) at
-// (kz / 2) ssb + kz % 2 + ix srs, blocked likewise.
+// A line packs the two x rows of its group's pair as real and imaginary parts.  Point (ix, iz)
+// of a field that both directions touch (p, Dx; acoustic also div, Lz) sits at (iz / 4) sb +
+// iz % 4 + ix rs: blocked (rs = 4, sb = 4 nxx), where an x pass's rows are contiguous and a CTA
+// of 4 z rows touches 64-byte pieces, or row by row (rs = nzz, sb = 4).  The fields of one
+// direction lie its way: the x pass's blocked, the z passes' row by row (rz = nzz).  Measured
+// with every field row by row: the x passes of a 1678 x 660 shot 45 against 32 us, 2461 x 860
+// 161 against 94; with every field blocked the z passes lose more than that.  Half spectra:
+// (ix, kz) at (kz / 2) ssb + kz % 2 + ix srs, blocked likewise.
 #pragma once
 #include "rt_kernels.cuh"
 
 namespace qp {
 
-// 2W rows of a field at address i of the first, nr of them on the grid.  Loads take rs = 0 when
-// not all are (a missing row then repeats the first one, which keeps its line finite).
-__device__ __forceinline__ Cx<float> ld_rows(const float* __restrict__ f, unsigned i, unsigned rs, Cx<float>*) {
+// Two rows of a field at address i of the first, nr of them on the grid.  Loads take rs = 0 when
+// the second is not (it then repeats the first one, which keeps its line finite).
+__device__ __forceinline__ Cx<float> ld_rows(const float* __restrict__ f, unsigned i, unsigned rs) {
     return {f[i], f[i + rs]};
-}
-__device__ __forceinline__ Cx<float2> ld_rows(const float* __restrict__ f, unsigned i, unsigned rs, Cx<float2>*) {
-    return {make_float2(f[i], f[i + rs]), make_float2(f[i + 2 * rs], f[i + 3 * rs])};
 }
 __device__ __forceinline__ void st_rows(float* f, unsigned i, unsigned rs, int nr, Cx<float> c) {
     f[i] = c.x;
     if (nr > 1) f[i + rs] = c.y;
 }
-__device__ __forceinline__ void st_rows(float* f, unsigned i, unsigned rs, int nr, Cx<float2> c) {
-    f[i] = c.x.x;
-    if (nr > 1) f[i + rs] = c.x.y;
-    if (nr > 2) f[i + 2 * rs] = c.y.x;
-    if (nr > 3) f[i + 3 * rs] = c.y.y;
-}
 
 // A thread's share of a z pass: its rows, and the loops over its points.
 template <class LR> struct ZRows {
+    static_assert(LR::W == 1, "a group's line holds one pair of rows");
     using C = typename LR::C;
-    static constexpr int NR = 2 * LR::W, NZ = LR::NZ;
+    static constexpr int NR = 2, NZ = LR::NZ;
     int n, x0, nr;
     unsigned rs, sb, rz;   // strides
     unsigned ls, lz;       // row strides of loads (0 when rows are missing)
@@ -67,9 +58,9 @@ template <class LR> struct ZRows {
         return (q >> 2) * sb + (q & 3) + (unsigned)x0 * rs;
     }
     __device__ __forceinline__ unsigned own(int r) const { return o0 + r * LR::B1; }
-    __device__ __forceinline__ C ld(const float* f, unsigned i) const { return ld_rows(f, i, ls, (C*)nullptr); }
+    __device__ __forceinline__ C ld(const float* f, unsigned i) const { return ld_rows(f, i, ls); }
     __device__ __forceinline__ void st(float* f, unsigned i, C c) const { st_rows(f, i, rs, nr, c); }
-    __device__ __forceinline__ C ldo(const float* f, unsigned i) const { return ld_rows(f, i, lz, (C*)nullptr); }
+    __device__ __forceinline__ C ldo(const float* f, unsigned i) const { return ld_rows(f, i, lz); }
     __device__ __forceinline__ void sto(float* f, unsigned i, C c) const { st_rows(f, i, rz, nr, c); }
     // use(r, q, i, o, load(i, o, q)) for this thread's points q = index(r), their addresses i in the
     // shared fields and o in the z passes' own; F: fields load reads
@@ -149,14 +140,8 @@ template <class LR> struct ZDft {
             const float sg = f < nzh ? 1.f : -1.f;
             const unsigned i = (unsigned)(k >> 1) * ssb + (k & 1) + (unsigned)z.x0 * srs;
             const unsigned rs = z.nr == ZRows<LR>::NR ? srs : 0;  // a missing row repeats the first
-            if constexpr (LR::W == 1) {
-                const float2 a = S[i], b = S[i + rs];
-                x[r] = {fmaf(-sg, b.y, a.x), fmaf(sg, a.y, b.x)};
-            } else {
-                const float2 a = S[i], b = S[i + rs], c = S[i + 2 * rs], d = S[i + 3 * rs];
-                x[r].x = make_float2(fmaf(-sg, c.y, a.x), fmaf(-sg, d.y, b.x));
-                x[r].y = make_float2(fmaf(sg, a.y, c.x), fmaf(sg, b.y, d.x));
-            }
+            const float2 a = S[i], b = S[i + rs];
+            x[r] = {fmaf(-sg, b.y, a.x), fmaf(sg, a.y, b.x)};
         }
     }
     // half spectra of the rows <- x, through the line buffer (barriers before, between and after)
@@ -179,15 +164,8 @@ template <class LR> struct ZDft {
                 auto put = [&](int row, float e0, float e1, float e2, float e3) {
                     if (row < z.nr) *reinterpret_cast<float4*>(o + row * srs) = make_float4(e0, e1, e2, e3);
                 };
-                if constexpr (LR::W == 1) {
-                    put(0, a0.x, a0.y, a1.x, a1.y);
-                    put(1, b0.x, b0.y, b1.x, b1.y);
-                } else {
-                    put(0, a0.x.x, a0.y.x, a1.x.x, a1.y.x);
-                    put(1, a0.x.y, a0.y.y, a1.x.y, a1.y.y);
-                    put(2, b0.x.x, b0.y.x, b1.x.x, b1.y.x);
-                    put(3, b0.x.y, b0.y.y, b1.x.y, b1.y.y);
-                }
+                put(0, a0.x, a0.y, a1.x, a1.y);
+                put(1, b0.x, b0.y, b1.x, b1.y);
             }
         __syncthreads();
     }
