@@ -15,7 +15,7 @@ size_t ac_xpass_smem(int L, int m, int nxx, int nstaged) {
 
 void launch_ac_zpass(const AcZArgs& a, cudaStream_t s) {
     if (a.pl.rt) {
-        rtz_any(a.pl.quick, [&](const RtzGroup& g) { return g.zpass(a, s); });
+        rtz_any(a.pl.quick, [&](const RtzGroup& g) { return g.zpass && g.zpass(a, s); });
         return;
     }
     const int grid = (a.nxx + 2 * a.L - 1) / (2 * a.L);

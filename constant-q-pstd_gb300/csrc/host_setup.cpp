@@ -325,7 +325,8 @@ static double mean_excess(const std::complex<double>* w, int n) {
 }
 
 static RtEntry entry(int id, RtAxis axis, bool quick) {
-    return axis == kRtX ? rt_entry(id, quick) : axis == kRtZ ? rtz_entry(id, quick) : RtEntry{};
+    if (axis == kRtX) return rt_entry(id, quick);
+    return axis == kRtZQ || (axis == kRtZ && id < kRtzVisco) ? rtz_entry(id, quick) : RtEntry{};
 }
 
 int rt_choose(int n, RtAxis axis) {
@@ -345,7 +346,8 @@ int rt_lines(int id, RtAxis axis, int quick) { return entry(id, axis, quick != 0
 int rt_length(int id, RtAxis axis) { return entry(id, axis, false).m; }
 
 // The quick form where the wide one would leave SMs without a CTA (one of several lines then
-// bounds the pass).  With the line at two CTAs per SM the 64-shot batch fell from 5.4 to 6.3 ms a
+// bounds the pass): fewer CTAs than the 152 SMs of the chip this is written for.  By the shot
+// alone, also in a batch or server.  With the line at two CTAs per SM the 64-shot batch fell from 5.4 to 6.3 ms a
 // step and the 1678 x 660 shot from 138.8 to 141.7 us; at half a CTA small grids lose up to 30 %.
 int rt_quick(int id, RtAxis axis, int lines) {
     const RtEntry w = entry(id, axis, false), q = entry(id, axis, true);

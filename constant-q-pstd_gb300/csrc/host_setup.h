@@ -37,7 +37,9 @@ int build_plan_host(int n, HostPlan& hp);
 // convolutions.  On an entry of rt_list.h's x or z passes (axis), where one is long
 // enough; else (or for kStockham) a Stockham plan, m = n when n factors into radices
 // <= 16, else a smooth m >= 2n-1.
-enum RtAxis { kStockham, kRtX, kRtZ };
+// kRtZQ: the z lines of the constant-Q step, which has entries of its own
+enum RtAxis { kStockham, kRtX, kRtZ, kRtZQ };
+inline RtAxis rt_zaxis(bool visco) { return visco ? kRtZQ : kRtZ; }
 int build_conv_plan_host(int n, HostPlan& hp, RtAxis axis = kStockham);
 // Is there a Stockham plan for an n-point line?
 bool stockham_line(int n);

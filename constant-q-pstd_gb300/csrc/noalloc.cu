@@ -58,7 +58,7 @@ __global__ void noalloc_coef_kernel(int N, float dt, const float* __restrict__ v
                                     float* c1, float* c2) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
-    // in double, rounded once, as qpstd_shot_create computes them on the host
+    // in double, rounded once, as ac_coef_kernel of qpstd_shot_create computes them
     const double v = vp[i], t = dt;
     c1[i] = (float)((double)rho[i] * v * v * t);
     c2[i] = (float)(v * v * t * t / 12.0);

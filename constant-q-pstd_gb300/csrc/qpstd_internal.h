@@ -212,7 +212,7 @@ struct VtabArgs {
 // Low-rank form of the constant-Q pressure term (qpstd_shot_set_lowrank):
 // x-spectral pass: per kz column, Q_b = F_x^-1[Vt_b F_x G] / (nxx nzz) for the
 // row factors b, as per-kz convolutions on the convolution plan (tables built
-// from V by vz_convtab_kernel, sym 4).
+// from V by convtab.cu, or by vz_convtab_kernel on Stockham plans).
 struct LrxArgs {
     int nxx, nzh, L, row;
     FFTPlanDev plc;

@@ -17,6 +17,7 @@ struct RtGroup {
     bool (*xexact)(const VxsArgs& a, cudaStream_t s);
     int (*limits)();
 };
+// (zpass: null in the groups of the constant-Q step alone)
 struct RtzGroup {
     bool (*zpass)(const AcZArgs& a, cudaStream_t s);
     bool (*passA)(const VzArgsA& a, cudaStream_t s);

@@ -67,8 +67,8 @@ template <class LR> constexpr int rt_batch(int F) {
     return u < 1 ? 1 : u > LR::NZ ? LR::NZ : u;
 }
 // use(r, ix, i, load(i, ix)) for this thread's rows r (ix = index(r) < n), the loads of U
-// rows in flight before the first use.  Offsets are 32 bits: the lines these passes plan (up to
-// about 4600 by 2800 points) stay far below 2^32 elements.
+// rows in flight before the first use.  Offsets are 32 bits: the windows these passes run (up to
+// 4608 points wide and, with z on a Stockham plan, up to 6561 deep) stay far below 2^32 elements.
 template <class LR, int U, class LoadF, class UseF>
 __device__ __forceinline__ void rt_rows(int n, unsigned pitch, unsigned off, bool on, LoadF&& load, UseF&& use) {
     using In = decltype(load(off, 0));

@@ -15,7 +15,19 @@
 // z entries are X(ID, W, PAD, GF, G, MB, R1, R2, R3, COST): PAD 0 transforms lines of exactly
 // M points, PAD 1 serves n <= (M + 1) / 2 (operators as padded convolutions, exact DFTs by
 // Bluestein's identity).  GF 1: a warp's threads are neighbouring rows, whose points are
-// neighbours in the blocked fields.
+// neighbours in the blocked fields.  The COSTs of the z entries decide nothing: at every depth the
+// shortest entry that fits has the least M x COST.
+//
+// The exact lengths up to entry 9 are the depths of the programs' standard models (160 + 2 x 10,
+// 160 + 2 x 20, 600 + 2 x 30) and a ladder of smooth depths from 256 to 800.  Those from entry 25 on
+// serve the constant-Q step alone: they are smooth depths where its batches ran slower padded (ten
+// roundtrips of more than 2n points a step) than on a direct Stockham transform.  16 shots 1300 to
+// 1855 wide, us a step, Stockham / padded / exact: 600 deep 1986 / 2354 / 1379, 768 2284 / 2575 /
+// 1652, 900 2717 / 2851 / 2026, 1728 5530 / 5714 / 3657.  Up to 384 points padded is faster than
+// Stockham, and at the smooth depths left out (490, 504, 972, 1152, 1400, 1500) within 8 % of it.
+// They have no quick form: lone shots 150 to 1000 wide take 0.54 to 1.03 of the padded forms' time.
+// An acoustic step (three roundtrips along z) is faster padded than Stockham at all of them, and a
+// lone one 1000 x 480 faster than exact too (23.6 against 29.2 us).
 //
 // The wide forms fill the chip with many lines; the quick forms have the same lengths with
 // fewer lines per CTA on more threads, for grids whose wide form has fewer CTAs than the
@@ -47,29 +59,45 @@
 #define QP_RTZ_G8(X) X(20, 1, 1, 0, 1, 4, 16, 10, 16, 1250) X(21, 1, 1, 0, 1, 3, 16, 12, 16, 1250)
 #define QP_RTZ_G9(X) X(22, 1, 1, 0, 1, 2, 16, 16, 16, 1150) X(23, 1, 1, 0, 1, 2, 16, 20, 16, 1140)
 #define QP_RTZ_G10(X) X(24, 1, 1, 0, 1, 1, 24, 16, 16, 1400)
-#define QP_RTZ_G11(X) X(1, 1, 0, 0, 1, 4, 5, 6, 6, 0) X(2, 1, 0, 0, 1, 4, 5, 5, 8, 0) X(3, 1, 0, 0, 1, 4, 8, 4, 8, 0) X(4, 1, 0, 0, 1, 4, 8, 5, 8, 0) X(5, 1, 0, 0, 1, 4, 10, 5, 8, 0)
-#define QP_RTZ_G12(X) X(6, 1, 0, 0, 1, 4, 8, 8, 8, 0) X(7, 1, 0, 0, 1, 4, 8, 8, 10, 0) X(8, 1, 0, 0, 1, 4, 11, 6, 10, 0) X(9, 1, 0, 0, 1, 4, 10, 8, 10, 0)
-#define QP_RTZ_G13(X) X(10, 1, 1, 0, 1, 4, 8, 4, 5, 0) X(11, 1, 1, 0, 1, 4, 8, 4, 8, 0) X(12, 1, 1, 0, 1, 4, 8, 6, 8, 0) X(13, 1, 1, 0, 1, 4, 8, 8, 8, 0)
-#define QP_RTZ_G14(X) X(14, 1, 1, 0, 1, 4, 8, 12, 8, 0) X(15, 1, 1, 0, 1, 4, 8, 16, 8, 0)
+#define QP_RTZ_G11(X) X(25, 1, 0, 1, 2, 5, 8, 6, 10, 1200) X(26, 1, 0, 1, 2, 5, 10, 5, 10, 1200) X(27, 1, 0, 1, 2, 5, 9, 6, 10, 1200)
+#define QP_RTZ_G12(X) X(28, 1, 0, 1, 2, 4, 8, 7, 10, 1200) X(29, 1, 0, 1, 2, 5, 10, 6, 10, 1200) X(30, 1, 0, 1, 2, 4, 10, 7, 10, 1200)
+#define QP_RTZ_G13(X) X(31, 1, 0, 1, 2, 4, 9, 8, 10, 1200) X(32, 1, 0, 1, 2, 3, 8, 12, 8, 1200) X(33, 1, 0, 1, 2, 3, 10, 7, 12, 1200)
+#define QP_RTZ_G14(X) X(34, 1, 0, 1, 2, 3, 10, 9, 10, 1200) X(35, 1, 0, 1, 2, 3, 10, 8, 12, 1200)
+#define QP_RTZ_G15(X) X(36, 1, 0, 1, 2, 2, 10, 7, 14, 1200) X(37, 1, 0, 1, 2, 2, 10, 10, 10, 1200) X(38, 1, 0, 1, 2, 2, 8, 16, 8, 1200)
+#define QP_RTZ_G16(X) X(39, 1, 0, 1, 2, 5, 7, 7, 8, 1200) X(40, 1, 0, 1, 2, 5, 10, 6, 7, 1200) X(41, 1, 0, 1, 2, 5, 8, 6, 9, 1200) X(42, 1, 0, 1, 2, 5, 8, 7, 8, 1200) X(43, 1, 0, 1, 2, 5, 10, 5, 9, 1200)
+#define QP_RTZ_G17(X) X(44, 1, 0, 1, 2, 4, 8, 8, 9, 1200) X(45, 1, 0, 1, 2, 3, 7, 7, 12, 1200) X(46, 1, 0, 1, 2, 4, 10, 7, 9, 1200) X(47, 1, 0, 1, 2, 4, 9, 8, 9, 1200) X(48, 1, 0, 1, 2, 3, 8, 7, 12, 1200)
+#define QP_RTZ_G18(X) X(49, 1, 0, 1, 2, 2, 8, 7, 14, 1200) X(50, 1, 0, 1, 2, 3, 9, 9, 10, 1200) X(51, 1, 0, 1, 2, 3, 9, 8, 12, 1200) X(52, 1, 0, 1, 2, 2, 9, 7, 14, 1200) X(53, 1, 0, 1, 2, 2, 8, 8, 14, 1200)
+#define QP_RTZ_G19(X) X(54, 1, 0, 1, 2, 2, 10, 7, 15, 1200) X(55, 1, 0, 1, 2, 2, 10, 9, 12, 1200) X(56, 1, 0, 1, 2, 2, 10, 8, 14, 1200) X(57, 1, 0, 1, 2, 2, 12, 9, 12, 1200) X(58, 1, 0, 1, 2, 2, 12, 8, 14, 1200)
+#define QP_RTZ_G20(X) X(59, 1, 0, 0, 1, 4, 10, 10, 16, 1200) X(60, 1, 0, 0, 1, 4, 12, 10, 14, 1200) X(61, 1, 0, 0, 1, 4, 12, 12, 12, 1200) X(62, 1, 0, 0, 1, 4, 16, 8, 14, 1200) X(63, 1, 0, 0, 1, 4, 12, 10, 15, 1200)
+#define QP_RTZ_G21(X) X(1, 1, 0, 0, 1, 4, 5, 6, 6, 0) X(2, 1, 0, 0, 1, 4, 5, 5, 8, 0) X(3, 1, 0, 0, 1, 4, 8, 4, 8, 0) X(4, 1, 0, 0, 1, 4, 8, 5, 8, 0) X(5, 1, 0, 0, 1, 4, 10, 5, 8, 0)
+#define QP_RTZ_G22(X) X(6, 1, 0, 0, 1, 4, 8, 8, 8, 0) X(7, 1, 0, 0, 1, 4, 8, 8, 10, 0) X(8, 1, 0, 0, 1, 4, 11, 6, 10, 0) X(9, 1, 0, 0, 1, 4, 10, 8, 10, 0)
+#define QP_RTZ_G23(X) X(10, 1, 1, 0, 1, 4, 8, 4, 5, 0) X(11, 1, 1, 0, 1, 4, 8, 4, 8, 0) X(12, 1, 1, 0, 1, 4, 8, 6, 8, 0) X(13, 1, 1, 0, 1, 4, 8, 8, 8, 0)
+#define QP_RTZ_G24(X) X(14, 1, 1, 0, 1, 4, 8, 12, 8, 0) X(15, 1, 1, 0, 1, 4, 8, 16, 8, 0)
 #define QP_RT_WIDE_ALL(X) \
     QP_RT_G0(X) QP_RT_G1(X) QP_RT_G2(X) QP_RT_G3(X) QP_RT_G4(X) QP_RT_G5(X) QP_RT_G6(X) QP_RT_G7(X) QP_RT_G8(X)
 #define QP_RT_QUICK_ALL(X) \
     QP_RT_G9(X) QP_RT_G10(X) QP_RT_G11(X) QP_RT_G12(X)
 #define QP_RTZ_WIDE_ALL(X) \
-    QP_RTZ_G0(X) QP_RTZ_G1(X) QP_RTZ_G2(X) QP_RTZ_G3(X) QP_RTZ_G4(X) QP_RTZ_G5(X) QP_RTZ_G6(X) QP_RTZ_G7(X) QP_RTZ_G8(X) QP_RTZ_G9(X) QP_RTZ_G10(X)
+    QP_RTZ_G0(X) QP_RTZ_G1(X) QP_RTZ_G2(X) QP_RTZ_G3(X) QP_RTZ_G4(X) QP_RTZ_G5(X) QP_RTZ_G6(X) QP_RTZ_G7(X) QP_RTZ_G8(X) QP_RTZ_G9(X) QP_RTZ_G10(X) \
+    QP_RTZ_G11(X) QP_RTZ_G12(X) QP_RTZ_G13(X) QP_RTZ_G14(X) QP_RTZ_G15(X) QP_RTZ_G16(X) QP_RTZ_G17(X) QP_RTZ_G18(X) QP_RTZ_G19(X) QP_RTZ_G20(X)
 #define QP_RTZ_QUICK_ALL(X) \
-    QP_RTZ_G11(X) QP_RTZ_G12(X) QP_RTZ_G13(X) QP_RTZ_G14(X)
+    QP_RTZ_G21(X) QP_RTZ_G22(X) QP_RTZ_G23(X) QP_RTZ_G24(X)
 // groups of the wide forms come first
 #define QP_RT_NWIDE 9
 #define QP_RT_NGROUPS 13
-#define QP_RTZ_NWIDE 11
-#define QP_RTZ_NGROUPS 15
+#define QP_RTZ_NWIDE 21
+// of which those from here on serve the constant-Q step alone
+#define QP_RTZ_NBOTH 11
+#define QP_RTZ_NGROUPS 25
 
 // Registers that an epilogue loop's loads in flight may take.  Wide z passes: 36 at 96 registers a
-// thread, four CTAs per SM (z passes of a 4100 x 660 shot 119 us; 24: 121; three CTAs of 128
-// registers 132, which a lone 1678 x 660 shot would like better, 62 against 64.5, and the 64-shot
-// batch worse, 5.68 against 5.36 ms).  Wide x passes: 24 (36 spills on the longest lines: x pass of
-// 4100 x 660 91 -> 99 us).  Quick: registers are plenty and each round of loads is a wait.
+// thread, four CTAs per SM (z passes of a 4100 x 660 constant-Q shot 119 us; 24: 121; three CTAs of
+// 128 registers 132, which a lone 1678 x 660 shot would like better, 62 against 64.5, and the
+// 64-shot batch worse, 5.68 against 5.36 ms).  Acoustic z passes of 1700- and 2500-wide shots, us at
+// 36 and at 24: 512 points 18.0 and 18.4, 600 39.6 and 41.5, 661 42.3 and 44.3, 768 47.9 and 49.6,
+// 1024 58.0 and 59.5, 2000 104.9 and 107; slower at 400 (18.0 and 16.8), 660 (31.4 and 30.3), both
+// of which spill at 36, and at 1200 (74.6 and 70.5).  Wide x passes: 24 (36 spills on the longest
+// lines: x pass of 4100 x 660 91 -> 99 us).  Quick: registers are plenty and each round of loads is a wait.
 constexpr int kEpiWide = 24, kEpiWideZ = 36, kEpiQuick = 96;
 
 // An entry's complex lines per CTA, length and radices (m = 0: no such entry).
@@ -98,4 +126,5 @@ inline RtEntry rtz_entry(int id, bool quick) {
 #undef QP_RT_CASE
     return {0, 0, 0, 0, 0, 0, 0};
 }
-constexpr int kRtIds = 19, kRtzIds = 24;
+constexpr int kRtIds = 19, kRtzIds = 63;
+constexpr int kRtzVisco = 25;  // z entries from here on serve the constant-Q step alone

@@ -14,6 +14,9 @@ template <class LR> unsigned z_grid(int nxx) { return (nxx + 2 * LR::G * LR::W -
 // passes with a second buffer (running sums)
 template <class LR> constexpr size_t smem_sum() { return LR::kSmem + LR::kLines; }
 
+// entries of the constant-Q step alone have no acoustic pass
+#define QP_RTZ_VISCO (QP_RTZ_GROUP >= QP_RTZ_NBOTH && QP_RTZ_GROUP < QP_RTZ_NWIDE)
+
 #define QP_RTZ_SWITCH(ID_OF, CASE) \
     switch (ID_OF) {               \
         QP_RTZ_ENTRIES(CASE)       \
@@ -27,7 +30,9 @@ template <class LR> constexpr size_t smem_sum() { return LR::kSmem + LR::kLines;
         using LR = LineRT<W, PAD, GF, G, MB, R1, R2, R3, (QP_RTZ_GROUP < QP_RTZ_NWIDE ? kEpiWideZ : kEpiQuick)>;                                                              \
         launch_rt(K<LR>, z_grid<LR>(a.nxx), LR::kThreads, SMEM, s, a.pl.pdl, a);                                                       \
     }
+#if !QP_RTZ_VISCO
 QP_RTZ_LAUNCH(zpass, AcZArgs, rt_zpass_kernel, LR::kSmem)
+#endif
 QP_RTZ_LAUNCH(passA, VzArgsA, rt_passA_kernel, LR::kSmem)
 QP_RTZ_LAUNCH(passB, VzArgsB, rt_passB_kernel, smem_sum<LR>())
 QP_RTZ_LAUNCH(passC, VzArgsC, rt_passC_kernel, LR::kSmem)
@@ -39,16 +44,24 @@ template <class K> bool up(K k, size_t bytes) {
 template <int W, bool PAD, bool GF, int G, int MB, int R1, int R2, int R3> int l_limits() {
     using LR = LineRT<W, PAD, GF, G, MB, R1, R2, R3, (QP_RTZ_GROUP < QP_RTZ_NWIDE ? kEpiWideZ : kEpiQuick)>;
     static_assert(smem_sum<LR>() <= QP_SMEM_DYN_MAX, "lines of an entry fit a CTA's shared memory");
-    return up(rt_zpass_kernel<LR>, LR::kSmem) | up(rt_passA_kernel<LR>, LR::kSmem) | up(rt_passB_kernel<LR>, smem_sum<LR>()) |
-           up(rt_passC_kernel<LR>, LR::kSmem) | up(rt_zsum_kernel<LR>, smem_sum<LR>());
+    bool bad = up(rt_passA_kernel<LR>, LR::kSmem) | up(rt_passB_kernel<LR>, smem_sum<LR>()) |
+               up(rt_passC_kernel<LR>, LR::kSmem) | up(rt_zsum_kernel<LR>, smem_sum<LR>());
+#if !QP_RTZ_VISCO
+    bad |= up(rt_zpass_kernel<LR>, LR::kSmem);
+#endif
+    return bad;
 }
 
+#if QP_RTZ_VISCO
+constexpr bool (*g_zpass)(const AcZArgs&, cudaStream_t) = nullptr;
+#else
 bool g_zpass(const AcZArgs& a, cudaStream_t s) {
 #define C_(ID, W, PAD, GF, G, MB, R1, R2, R3, COST) \
     case ID: l_zpass<W, PAD, GF, G, MB, R1, R2, R3>(a, s); break;
     QP_RTZ_SWITCH(a.pl.rt, C_)
 #undef C_
 }
+#endif
 bool g_passA(const VzArgsA& a, cudaStream_t s) {
 #define C_(ID, W, PAD, GF, G, MB, R1, R2, R3, COST) \
     case ID: l_passA<W, PAD, GF, G, MB, R1, R2, R3>(a, s); break;

@@ -372,7 +372,7 @@ static int setup_plain(qpstd_shot* s, const qpstd_shot_desc* d) {
 // separable operators (two staggered derivatives and the k^2 term per axis).
 static int setup_conv(qpstd_shot* s, const qpstd_shot_desc* d) {
     HostPlan cx, cz;
-    if (build_conv_plan_host(d->nxx, cx, kRtX) || build_conv_plan_host(d->nzz, cz, s->blk ? kRtZ : kStockham))
+    if (build_conv_plan_host(d->nxx, cx, kRtX) || build_conv_plan_host(d->nzz, cz, s->blk ? rt_zaxis(s->visco) : kStockham))
         return fail(QPSTD_ENOTSUP, "no convolution plan for this length");
     // the forms of the passes: their tables take back the gain of the form's roundtrip
     const int pairs_x = (d->nzz + 1) / 2, pairs_z = (d->nxx + 1) / 2;
@@ -380,7 +380,7 @@ static int setup_conv(qpstd_shot* s, const qpstd_shot_desc* d) {
         s->qx = rt_quick(cx.rt, kRtX, pairs_x);
         s->qs = rt_quick(cx.rt, kRtX, s->nzh);
     }
-    if (cz.rt) s->qz = rt_quick(cz.rt, kRtZ, pairs_z);
+    if (cz.rt) s->qz = rt_quick(cz.rt, rt_zaxis(s->visco), pairs_z);
     // z transforms on an entry's own length, forward in one pass and inverse in another: what
     // happens between them takes back their gain
     const double zgain = cz.rt && cz.m == cz.n ? cz.gain[s->qz] : 0.0;
@@ -608,7 +608,7 @@ int shot_create_ex(const qpstd_shot_desc* d, qpstd_shot** out, bool tune, qp::Ar
         if (s->stage_z && (size_t)8 * s->pzc.m + stz > 110 * 1024) s->Lzp = 1;
         // constant-Q: z pass B and the 3-output x-spectral pass hold two line buffers;
         // z pass A uses both the exact and the convolution plan
-        s->Lzv = s->pzc.rt ? rt_lines(s->pzc.rt, kRtZ, s->qz) : choose_L(pairs_z, std::max(s->pz.m, s->pzc.m), std::max(s->pz.tx, s->pzc.tx), 2, false);
+        s->Lzv = s->pzc.rt ? rt_lines(s->pzc.rt, rt_zaxis(s->visco), s->qz) : choose_L(pairs_z, std::max(s->pz.m, s->pzc.m), std::max(s->pz.tx, s->pzc.tx), 2, false);
         if (!s->px.rt) {
             s->Lxs = choose_L(s->nzh, s->px.m, s->px.tx, 1, true);
             s->Lxs3 = choose_L(s->nzh, s->px.m, s->px.tx, 2, true);
@@ -869,8 +869,8 @@ static void plain_one(qpstd_shot* s, Wave& w, float src, int t_filter, float eta
 // quarter ulp of ka, which with the reference's eta ~ 1e-26 holds for every
 // step of ordinary runs.  The correction grows with tt, so per eta the largest
 // such step is found once (over 4096 samples of ka up to the grid's largest);
-// steps up to it use the k^1.01 operator -- the per-kz convolution when the
-// width needs Bluestein -- instead of exact transforms.
+// steps up to it use the k^1.01 operator -- the per-kz convolution -- instead of
+// exact transforms.
 static bool filter_is_ka(qpstd_shot* s, float eta, int t) {
     for (auto& c : s->ka_steps)
         if (c.first == eta) return t <= c.second;
@@ -1296,14 +1296,14 @@ extern "C" long long qpstd_shot_bytes(const qpstd_shot_desc* d) {
     const bool visco = d->kind == QPSTD_VAPS || d->kind == QPSTD_QRTM;
     const bool rtm = d->kind == QPSTD_ARTM || d->kind == QPSTD_QRTM;
     const bool fused = d->method != QPSTD_PLAIN;
-    const int ix = rt_choose(d->nxx, kRtX), iz = ix && stockham_line(d->nzz) ? rt_choose(d->nzz, kRtZ) : 0;
+    const int ix = rt_choose(d->nxx, kRtX), iz = ix && stockham_line(d->nzz) ? rt_choose(d->nzz, rt_zaxis(visco)) : 0;
     const bool blk = fused && iz;
     const double Nu = (double)d->nxx * d->nzz, N = blk ? (double)d->nxx * ((d->nzz + 3) / 4 * 4) : Nu;
     const double nzh = (d->nzz / 2 + 2) & ~1, NS = d->nxx * nzh;
     const double nr = std::max(d->nr, 1), nx = d->nxx - 2 * d->pml, nz = d->nzz - 2 * d->pml;
     HostPlan cx, cz, ex, ez;
     if (ix) cx.m = ex.m = rt_length(ix, kRtX);
-    if (iz) cz.m = ez.m = rt_length(iz, kRtZ);
+    if (iz) cz.m = ez.m = rt_length(iz, rt_zaxis(visco));
     if (fused && ((!ix && (build_conv_plan_host(d->nxx, cx) || build_plan_host(d->nxx, ex))) ||
                   (!iz && (build_conv_plan_host(d->nzz, cz) || build_plan_host(d->nzz, ez)))))
         return -1;  // no fused plan for these lengths

@@ -36,6 +36,16 @@ def test_wide_z_entries(kind, nxx, nzz):
     _check(kind, nxx, nzz, steps=2)
 
 
+# depths with an entry of their own for the constant-Q step and no quick form (acoustic: padded); a
+# last group with one row, with a full pair
+@pytest.mark.parametrize("nzz", [392, 420, 432, 448, 450, 480, 500, 540, 560, 576, 588, 600, 630, 648, 672, 700, 720, 768,
+                                 784, 810, 840, 864, 882, 896, 900, 960, 980, 1000, 1024, 1050, 1080, 1120, 1296, 1344,
+                                 1600, 1680, 1728, 1792, 1800])
+@pytest.mark.parametrize("kind,nxx", [(qpstd.APS, 41), (qpstd.VAPS, 41), (qpstd.VAPS, 42)])
+def test_exact_depths(kind, nxx, nzz):
+    _check(kind, nxx, nzz, steps=2)
+
+
 # x on an entry and z on a Stockham plan; both on Stockham plans
 @pytest.mark.parametrize("nxx,nzz", [(60, 3200), (61, 3201), (70, 3074), (5040, 42), (5040, 60)])
 @pytest.mark.parametrize("kind", KINDS)
